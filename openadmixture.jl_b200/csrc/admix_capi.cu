@@ -47,6 +47,8 @@ struct admix_ctx {
     double *U = nullptr, *V = nullptr, *vt = nullptr;
     int32_t *status_q = nullptr, *status_p = nullptr;
     uint8_t *pkg = nullptr;          /* mixed sweeps: per-chunk packages of the fixed block */
+    double *dump = nullptr;          /* expanded sums of admix_grad_hess_* (kept up to DUMP_KEEP bytes) */
+    size_t dump_bytes = 0;
     double *mu = nullptr;            /* ADMIX_FLAG_MEAN_IMPUTE: the SNP means g.mu (J) */
     double *ll_partial = nullptr, *qn_partial = nullptr;
     DevScalars *sc = nullptr;
@@ -55,7 +57,7 @@ struct admix_ctx {
     unsigned long long *counts = nullptr;
     LoglikPlan llp;
     SweepPlan sq, sp, sqm, spm, llm; /* *m: mixed-precision Q sweep, P sweep, loglik */
-    int64_t cap_sqm = 1, cap_spm = 1, cap_llm = 1;   /* slice counts the partial buffers hold */
+    int64_t cap_sq = 1, cap_sp = 1, cap_sqm = 1, cap_spm = 1, cap_llm = 1;   /* slice counts the partial buffers hold */
     QNPlan qnp;
     size_t bytes = 0;
     cudaGraphExec_t iter_graph = nullptr;
@@ -136,7 +138,7 @@ static void release(admix_ctx *h)
     if (h->cst) { cudaStreamSynchronize(h->cst); cudaStreamDestroy(h->cst); }
     if (h->host_registered) cudaHostUnregister((void *)h->host_bed);
     void *dps[] = {h->pkg, h->xbuf, h->parts_q, h->parts_p, h->U, h->V, h->vt, h->status_q,
-                   h->status_p, h->ll_partial, h->qn_partial, h->sc, h->counts, h->mu};
+                   h->status_p, h->ll_partial, h->qn_partial, h->sc, h->counts, h->mu, h->dump};
     for (void *p : dps)
         if (p) cudaFree(p);
     if (h->sc_host) cudaFreeHost(h->sc_host);
@@ -208,6 +210,8 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     h->spm = plan_sweep_p_mixed(K, I, J, h->sms);
     h->llm = plan_loglik_mixed(K, I, J, h->sms);
     h->qnp = plan_qn(nx, h->sms);
+    h->cap_sq = h->sq.S;
+    h->cap_sp = h->sp.S;
     h->cap_sqm = h->sqm.S;
     h->cap_spm = h->spm.S;
     h->cap_llm = h->llm.S;
@@ -254,9 +258,9 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     auto ll_parts = [&](int64_t nj) {
         const LoglikPlan a = plan_loglik(I, nj, h->sms);
         const SweepPlan b = plan_loglik_mixed(K, I, nj, h->sms);
-        return std::max((size_t)a.gx * a.gy, (size_t)b.gx * b.S);
+        return std::max((size_t)a.gx, (size_t)b.gx * b.S);
     };
-    size_t n_ll = std::max((size_t)h->llp.gx * h->llp.gy, (size_t)h->llm.gx * h->llm.S);
+    size_t n_ll = std::max((size_t)h->llp.gx, (size_t)h->llm.gx * h->llm.S);
     if (h->streamed)
         n_ll = std::max(n_ll, std::max(ll_parts(std::min<int64_t>(h->blk, J)), ll_parts(J - (int64_t)(h->nblk - 1) * h->blk)));
     TRY(dalloc(h, &h->ll_partial, n_ll));
@@ -426,7 +430,7 @@ static cudaError_t enq_loglik(admix_ctx *h, int which, double *dst, bool fast = 
                                        &h->sc->tc_err, h->pkg, h->st);
         }
         const LoglikPlan pl = h->streamed ? plan_loglik(h->I, nj, h->sms) : h->llp;
-        return launch_loglik_f64(h->K, bed, h->I, nj, h->pitch, Qof(h, which), P, pl, h->ll_partial, o, h->st, h->mu);
+        return launch_loglik_f64(h->K, bed, h->I, nj, h->pitch, Qof(h, which), P, pl, true, h->ll_partial, o, h->st, h->mu);
     };
     cudaError_t e = for_blocks(h, one);
     if (e == cudaSuccess && h->streamed) e = launch_sum_doubles(h->ll_blk, h->nblk, dst, h->st);
@@ -473,7 +477,7 @@ static cudaError_t enq_sweep_p_mode(admix_ctx *h, int mode, int wq, int wp, int 
             return launch_sweep_p_mixed(h->K, mode == 2 ? 1 : 0, bed, h->I, nj, h->pitch, Qof(h, wq), P, pl, out,
                                         &h->sc->tc_err, h->pkg, h->st);
         }
-        const SweepPlan pl = h->streamed ? block_plan(plan_sweep_p(h->K, h->I, nj, h->sms), (h->I + 3) / 4 * 4) : h->sp;
+        const SweepPlan pl = h->streamed ? block_plan(plan_sweep_p(h->K, h->I, nj, h->sms), (h->I + 31) / 32 * 32) : h->sp;
         return launch_sweep_p_f64(h->K, mode, bed, h->I, nj, h->pitch, Qof(h, wq), P, pl, out, h->st, h->mu);
     });
 }
@@ -646,33 +650,43 @@ int admix_init_em(admix_ctx *h, int32_t iters, double *ll_hist)
     return tc_err_sync(h);
 }
 
+/* The dump buffer stays with the handle unless it is large: allocating and freeing it in every call cost
+ * 0.1 to 1.2 ms, depending on whether the allocator had to map memory. */
+static const size_t DUMP_KEEP = (size_t)256 << 20;
+
 static int grad_hess_common(admix_ctx *h, bool qside, int32_t wq, int32_t wp, double *XtX, double *Xtz)
 {
     if (!h) return fail(nullptr, ADMIX_ERR_ARG, "handle is NULL");
     if (!valid_which(wq) || !valid_which(wp)) return fail(h, ADMIX_ERR_ARG, "invalid buffer selector");
     const int64_t nprob = qside ? h->I : h->J;
     const int K = h->K;
-    double *d_XtX = nullptr, *d_Xtz = nullptr;
-    if (cudaMalloc((void **)&d_XtX, sizeof(double) * K * K * nprob) != cudaSuccess ||
-        cudaMalloc((void **)&d_Xtz, sizeof(double) * K * nprob) != cudaSuccess) {
-        if (d_XtX) cudaFree(d_XtX);
-        return fail(h, ADMIX_ERR_NOMEM, "dump buffers: cudaMalloc failed");
+    const size_t nX = (size_t)K * K * nprob, need = sizeof(double) * (nX + (size_t)K * nprob);
+    if (need > h->dump_bytes) {
+        if (h->dump) cudaFree(h->dump);
+        h->bytes -= h->dump_bytes;
+        h->dump = nullptr;
+        h->dump_bytes = 0;
+        if (cudaMalloc((void **)&h->dump, need) != cudaSuccess) {
+            h->dump = nullptr;
+            cudaGetLastError();
+            return fail(h, ADMIX_ERR_NOMEM, "dump buffers: cudaMalloc failed");
+        }
+        h->dump_bytes = need;
+        h->bytes += need;
     }
-    cudaError_t e;
-    if (qside) {
-        int S = 1;
-        e = enq_sweep_q(h, wq, wp, &S);
-        if (e == cudaSuccess) e = launch_expand_hess(nprob, K, S, h->parts_q, d_XtX, d_Xtz, h->sms, h->st);
-    } else {
-        int S = 1;
-        e = enq_sweep_p(h, wq, wp, &S);
-        if (e == cudaSuccess) e = launch_expand_hess(nprob, K, S, h->parts_p, d_XtX, d_Xtz, h->sms, h->st);
-    }
-    if (e == cudaSuccess && XtX) e = cudaMemcpyAsync(XtX, d_XtX, sizeof(double) * K * K * nprob, cudaMemcpyDeviceToHost, h->st);
+    double *d_XtX = h->dump, *d_Xtz = h->dump + nX;
+    int S = 1;
+    cudaError_t e = qside ? enq_sweep_q(h, wq, wp, &S) : enq_sweep_p(h, wq, wp, &S);
+    if (e == cudaSuccess) e = launch_expand_hess(nprob, K, S, qside ? h->parts_q : h->parts_p, d_XtX, d_Xtz, h->sms, h->st);
+    if (e == cudaSuccess && XtX) e = cudaMemcpyAsync(XtX, d_XtX, sizeof(double) * nX, cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess && Xtz) e = cudaMemcpyAsync(Xtz, d_Xtz, sizeof(double) * K * nprob, cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-    cudaFree(d_XtX);
-    cudaFree(d_Xtz);
+    if (h->dump_bytes > DUMP_KEEP) {
+        cudaFree(h->dump);
+        h->bytes -= h->dump_bytes;
+        h->dump = nullptr;
+        h->dump_bytes = 0;
+    }
     if (e != cudaSuccess) return fail(h, ADMIX_ERR_CUDA, "grad/hess sweep failed: %s", cudaGetErrorString(e));
     return tc_err_sync(h);
 }
@@ -912,7 +926,7 @@ size_t admix_loglik_dev_workspace(int64_t I, int64_t J, int32_t K)
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const LoglikPlan pl = plan_loglik(I, J, sms);
-    return sizeof(double) * (size_t)pl.gx * pl.gy;
+    return sizeof(double) * (size_t)pl.gx;
 }
 
 int admix_loglik_dev(const uint8_t *d_bed, int64_t I, int64_t J, int32_t K, const double *d_q,
@@ -926,10 +940,10 @@ int admix_loglik_dev(const uint8_t *d_bed, int64_t I, int64_t J, int32_t K, cons
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return fail(nullptr, ADMIX_ERR_CUDA, "no current CUDA device");
     const LoglikPlan pl = plan_loglik(I, J, sms);
-    if (work_bytes < sizeof(double) * (size_t)pl.gx * pl.gy)
+    if (work_bytes < sizeof(double) * (size_t)pl.gx)
         return fail(nullptr, ADMIX_ERR_ARG, "workspace of %zu bytes is below the %zu required", work_bytes,
-                    sizeof(double) * (size_t)pl.gx * pl.gy);
-    cudaError_t e = launch_loglik_f64(K, d_bed, I, J, (I + 3) / 4, d_q, d_p, pl, (double *)d_work, d_out, (cudaStream_t)stream);
+                    sizeof(double) * (size_t)pl.gx);
+    cudaError_t e = launch_loglik_f64(K, d_bed, I, J, (I + 3) / 4, d_q, d_p, pl, false, (double *)d_work, d_out, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(nullptr, ADMIX_ERR_CUDA, "loglik launch failed: %s", cudaGetErrorString(e));
     return ADMIX_OK;
 }
@@ -986,13 +1000,13 @@ static void batch_release(admix_batch *b)
 }
 
 /* Plans of one member as if it had sms_eff SMs to itself.  The partial-sum buffers were sized
- * for the full SM count: the FP64 plans' slice counts only shrink with fewer SMs, and the mixed
- * plans are held to the slice counts of the handle's first plans. */
+ * for the full SM count, so the plans are held to the slice counts of the handle's first plans
+ * (the FP64 log-likelihood's partial sums are at most its CTAs, which only shrink). */
 static void set_plans(admix_ctx *h, int sms_eff)
 {
     h->llp = plan_loglik(h->I, h->J, sms_eff);
-    h->sq = plan_sweep_q(h->K, h->I, h->J, sms_eff);
-    h->sp = plan_sweep_p(h->K, h->I, h->J, sms_eff);
+    h->sq = plan_sweep_q(h->K, h->I, h->J, sms_eff, h->cap_sq);
+    h->sp = plan_sweep_p(h->K, h->I, h->J, sms_eff, h->cap_sp);
     h->sqm = plan_sweep_q_mixed(h->K, h->I, h->J, sms_eff, h->cap_sqm);
     h->spm = plan_sweep_p_mixed(h->K, h->I, h->J, sms_eff, h->cap_spm);
     h->llm = plan_loglik_mixed(h->K, h->I, h->J, sms_eff, h->cap_llm);

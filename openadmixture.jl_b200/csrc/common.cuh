@@ -84,10 +84,6 @@ __device__ __forceinline__ void project_simplex_local(double (&b)[K])
     for (int i = 0; i < K; ++i) b[i] = fmax(b[i] - tmax, 0.0) + pc;
 }
 
-/* sub-split of the per-problem accumulator list over NS threads, chosen by K so the
- * FP64 accumulators of one thread stay in registers. */
-__host__ __device__ constexpr int ns_for_k(int K) { return K <= 8 ? 1 : (K <= 12 ? 2 : 4); }
-
 #define ADMIX_DISPATCH_K(KV, CALL)                                              \
     switch (KV) {                                                               \
     case 1: { constexpr int KK = 1; CALL; } break;                              \

@@ -7,18 +7,24 @@
 #include <algorithm>
 #include "common.cuh"
 
-struct LoglikPlan { int gx = 1, gy = 1; int64_t jslice = 1; };
+/* gx CTAs (= partial sums) over nunit units: nblk blocks of 128 SNPs x slices of islice individuals */
+struct LoglikPlan { int gx = 1; int64_t nblk = 1, nunit = 1, islice = 32; };
 struct SweepPlan  { int gx = 1, S = 1; int64_t slice = 1; };
 
 LoglikPlan plan_loglik(int64_t I, int64_t J, int sms);
-SweepPlan plan_sweep_q(int K, int64_t I, int64_t J, int sms);
-SweepPlan plan_sweep_p(int K, int64_t I, int64_t J, int sms);
+/* Slices of the second axis for CTAs of 128 rows, per_sm of which are resident per SM: whole waves, slices
+ * a multiple of unit columns and at least min_units of them long, at most smax slices. */
+SweepPlan plan_rows(int64_t rows, int64_t cols, int sms, int per_sm, int64_t unit, int64_t min_units, int64_t smax);
+/* at most smax slices (a handle's partial-sum buffers are sized for its first plans) */
+SweepPlan plan_sweep_q(int K, int64_t I, int64_t J, int sms, int64_t smax = INT64_MAX);
+SweepPlan plan_sweep_p(int K, int64_t I, int64_t J, int sms, int64_t smax = INT64_MAX);
 
 /* FP64 sweeps (sweeps_f64.cu) */
 cudaError_t prepare_sweeps(int K);
-/* mu (J doubles, the SNP means) != nullptr selects the reference's non-skipmissing loops */
+/* mu (J doubles, the SNP means) != nullptr selects the reference's non-skipmissing loops.  padded: the
+ * handle's column layout (16-byte pitch, padding coded missing). */
 cudaError_t launch_loglik_f64(int K, const uint8_t *bed, int64_t I, int64_t J, int64_t pitch, const double *q,
-                              const double *p, const LoglikPlan &pl, double *partial, double *out,
+                              const double *p, const LoglikPlan &pl, bool padded, double *partial, double *out,
                               cudaStream_t st, const double *mu = nullptr);
 cudaError_t launch_sweep_q_f64(int K, int mode, const uint8_t *bed, int64_t I, int64_t J, int64_t pitch,
                                const double *q, const double *p, const SweepPlan &pl, double *out,

@@ -61,11 +61,13 @@ extern "C" int admix_loglik_dev_noalloc(const uint8_t *d_bed, int64_t I, int64_t
         return noalloc_fail(ADMIX_ERR_CUDA, "no current CUDA device");
     if (dev < 0 || dev >= kMaxDevices) return noalloc_fail(ADMIX_ERR_UNSUPPORTED, "device index beyond 63");
     const LoglikPlan pl = plan_loglik(I, J, sms);
-    const int64_t nparts = (int64_t)pl.gx * pl.gy;
-    if (nparts > ADMIX_NOALLOC_MAX_PARTIALS) {
+    /* the documented size limit, 1024 individuals per slot of the scratch; the plan itself needs no more
+     * slots than two per SM */
+    const int64_t groups = ((I + 3) / 4 + 255) / 256;
+    if (groups > ADMIX_NOALLOC_MAX_PARTIALS || pl.gx > ADMIX_NOALLOC_MAX_PARTIALS) {
         char buf[200];
-        snprintf(buf, sizeof(buf), "this cohort needs %lld partial sums; the static scratch holds %d "
-                 "(I up to about 33 million individuals)", (long long)nparts, ADMIX_NOALLOC_MAX_PARTIALS);
+        snprintf(buf, sizeof(buf), "this cohort needs %lld slots of 1024 individuals; the static scratch holds %d "
+                 "(I up to about 33 million individuals)", (long long)groups, ADMIX_NOALLOC_MAX_PARTIALS);
         return noalloc_fail(ADMIX_ERR_UNSUPPORTED, buf);
     }
     /* the runtime call above made the device's primary context current; the driver's
@@ -99,7 +101,7 @@ extern "C" int admix_loglik_dev_noalloc(const uint8_t *d_bed, int64_t I, int64_t
         }
         scratch = g_scratch[dev];
     }
-    cudaError_t e = launch_loglik_f64(K, d_bed, I, J, (I + 3) / 4, d_q, d_p, pl, (double *)scratch, d_out,
+    cudaError_t e = launch_loglik_f64(K, d_bed, I, J, (I + 3) / 4, d_q, d_p, pl, false, (double *)scratch, d_out,
                                       (cudaStream_t)stream);
     if (e != cudaSuccess) return noalloc_fail(ADMIX_ERR_CUDA, cudaGetErrorString(e));
     return ADMIX_OK;

@@ -1624,37 +1624,6 @@ size_t ll_pkg_bytes_t(int64_t I)
     return (size_t)((I + LT_IC - 1) / LT_IC) * LT<K>::PKG;
 }
 
-/* Slices over the second axis for CTAs of 128 rows, `per_sm` of which are resident per SM.  CTAs
- * of one launch take equal time, so the launch lasts ceil(gx S / (sms per_sm)) waves of CTAs that
- * each do 1/S of a row tile's work; S minimises waves / S, plus 0.5 % per extra slice (each adds a
- * partial slice for the consumer to read).  Slices are multiples of `unit`, at least 4 units
- * long, and at most smax. */
-SweepPlan plan_rows(int64_t rows, int64_t cols, int sms, int per_sm, int64_t unit, int64_t smax)
-{
-    SweepPlan pl;
-    pl.gx = (int)std::max<int64_t>(1, (rows + 127) / 128);
-    pl.S = 1;
-    pl.slice = std::max<int64_t>(unit, (cols + unit - 1) / unit * unit);
-    if (cols <= 0) return pl;
-    const int64_t cap = std::max<int64_t>(1, (int64_t)sms * per_sm);
-    const int64_t fill = (cap + pl.gx - 1) / pl.gx;   /* slices that fill the GPU once */
-    const int64_t top = std::min<int64_t>({std::max<int64_t>(1, (cols + 4 * unit - 1) / (4 * unit)),
-                                           std::max<int64_t>(16, 2 * fill), std::max<int64_t>(1, smax)});
-    double best = 1e300;
-    for (int64_t s = 1; s <= top; ++s) {
-        const int64_t slice = ((cols + s - 1) / s + unit - 1) / unit * unit;
-        const int64_t S = (cols + slice - 1) / slice;
-        const int64_t waves = ((int64_t)pl.gx * S + cap - 1) / cap;
-        const double cost = (double)waves / (double)S * (1.0 + 0.005 * (double)(S - 1));
-        if (cost < best - 1e-12) {
-            best = cost;
-            pl.S = (int)S;
-            pl.slice = slice;
-        }
-    }
-    return pl;
-}
-
 /* Resident CTAs per SM of one kernel, from its registers (allocated per warp in units of 256),
  * its static and dynamic shared memory (plus the per-CTA reservation), its threads and its tensor
  * memory columns (512 per SM).  The occupancy query answered one CTA per SM for all three mixed
@@ -1723,6 +1692,37 @@ int resident(int kind, int K, int fallback)
 
 } // namespace
 
+/* Slices over the second axis for CTAs of 128 rows, `per_sm` of which are resident per SM.  CTAs
+ * of one launch take equal time, so the launch lasts ceil(gx S / (sms per_sm)) waves of CTAs that
+ * each do 1/S of a row tile's work; S minimises waves / S, plus 0.5 % per extra slice (each adds a
+ * partial slice for the consumer to read).  Slices are multiples of `unit`, at least
+ * min_units units long, and at most smax. */
+SweepPlan plan_rows(int64_t rows, int64_t cols, int sms, int per_sm, int64_t unit, int64_t min_units, int64_t smax)
+{
+    SweepPlan pl;
+    pl.gx = (int)std::max<int64_t>(1, (rows + 127) / 128);
+    pl.S = 1;
+    pl.slice = std::max<int64_t>(unit, (cols + unit - 1) / unit * unit);
+    if (cols <= 0) return pl;
+    const int64_t cap = std::max<int64_t>(1, (int64_t)sms * per_sm);
+    const int64_t fill = (cap + pl.gx - 1) / pl.gx;   /* slices that fill the GPU once */
+    const int64_t top = std::min<int64_t>({std::max<int64_t>(1, (cols + min_units * unit - 1) / (min_units * unit)),
+                                           std::max<int64_t>(16, 2 * fill), std::max<int64_t>(1, smax)});
+    double best = 1e300;
+    for (int64_t s = 1; s <= top; ++s) {
+        const int64_t slice = ((cols + s - 1) / s + unit - 1) / unit * unit;
+        const int64_t S = (cols + slice - 1) / slice;
+        const int64_t waves = ((int64_t)pl.gx * S + cap - 1) / cap;
+        const double cost = (double)waves / (double)S * (1.0 + 0.005 * (double)(S - 1));
+        if (cost < best - 1e-12) {
+            best = cost;
+            pl.S = (int)S;
+            pl.slice = slice;
+        }
+    }
+    return pl;
+}
+
 cudaError_t prepare_mixed(int K)
 {
     cudaError_t e = cudaErrorInvalidValue;
@@ -1735,19 +1735,19 @@ cudaError_t prepare_mixed(int K)
  * split, and another split (batch autotuning) only regroups FP64 sums. */
 SweepPlan plan_sweep_q_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
 {
-    return plan_rows(I, J, sms, resident(0, K, 3), (int64_t)MX_DRAIN * MQ_JC, smax);
+    return plan_rows(I, J, sms, resident(0, K, 3), (int64_t)MX_DRAIN * MQ_JC, 4, smax);
 }
 
 /* One CTA per 128 SNPs and individual slice (slices are multiples of MX_DRAIN chunks, as above). */
 SweepPlan plan_sweep_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
 {
-    return plan_rows(J, I, sms, resident(1, K, 3), (int64_t)MX_DRAIN * MP_IC, smax);
+    return plan_rows(J, I, sms, resident(1, K, 3), (int64_t)MX_DRAIN * MP_IC, 4, smax);
 }
 
 /* One CTA per 128 SNPs and individual slice (slices are multiples of 32 individuals). */
 SweepPlan plan_loglik_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
 {
-    return plan_rows(J, I, sms, resident(2, K, 4), LT_IC, smax);
+    return plan_rows(J, I, sms, resident(2, K, 4), LT_IC, 4, smax);
 }
 
 cudaError_t launch_sweep_q_mixed(int K, const uint8_t *bed, int64_t I, int64_t J, int64_t pitch, const double *q,
