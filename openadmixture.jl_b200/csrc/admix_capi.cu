@@ -198,7 +198,6 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     TRYC(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->dev));
     TRYC(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
     TRYC(prepare_sweeps(K));
-    TRYC(prepare_qp(K));
     if (flags & ADMIX_FLAG_MIXED) TRYC(prepare_mixed(K));
 
     const int64_t nx = (int64_t)K * (I + J);

@@ -82,7 +82,6 @@ cudaError_t launch_loglik_mixed(int K, const uint8_t *bed, int64_t I, int64_t J,
 cudaError_t launch_mask_tail(uint8_t *bed, int64_t I, int64_t J, int64_t pitch, int sms, cudaStream_t st);
 
 /* batched QP + projection (qp_batch.cu) */
-cudaError_t prepare_qp(int K);
 cudaError_t launch_qp(int K, bool simplex, int64_t nprob, const double *parts, int S,
                       const double *x, double *x_next, int32_t *status, int32_t *fail_count,
                       const double *vt, int mu_mode, int damp_retry, cudaStream_t st);
