@@ -29,7 +29,6 @@ struct admix_ctx {
     int dev = 0, sms = 148;
     cudaStream_t st = nullptr;
     uint8_t *bed = nullptr;
-    bool owns_bed = true;            /* false for batch members: the batch owns the genotypes */
     /* out-of-core: the packed genotypes stay in the caller's (page-locked) host memory and every
      * pass streams SNP blocks of blk columns through two device buffers */
     bool streamed = false;
@@ -52,14 +51,17 @@ struct admix_ctx {
     double *mu = nullptr;            /* ADMIX_FLAG_MEAN_IMPUTE: the SNP means g.mu (J) */
     double *ll_partial = nullptr, *qn_partial = nullptr;
     DevScalars *sc = nullptr;
-    DevScalars *sc_host = nullptr;   /* pinned mirror */
-    int32_t *iter_host = nullptr;    /* pinned */
+    DevScalars sc_store = {};        /* host mirror of the scalars ... */
+    int32_t iter_store = 0;          /* ... and the iteration number to send */
+    DevScalars *sc_host = &sc_store; /* a batch points these at its pinned block (its graph copies them) */
+    int32_t *iter_host = &iter_store;
     unsigned long long *counts = nullptr;
     LoglikPlan llp;
     SweepPlan sq, sp, sqm, spm, llm; /* *m: mixed-precision Q sweep, P sweep, loglik */
     int64_t cap_sq = 1, cap_sp = 1, cap_sqm = 1, cap_spm = 1, cap_llm = 1;   /* slice counts the partial buffers hold */
     QNPlan qnp;
     size_t bytes = 0;
+    void *arena = nullptr;           /* one allocation for every device buffer but the dump's (a batch member's genotypes are the batch's) */
     cudaGraphExec_t iter_graph = nullptr;
     cudaGraph_t iter_graph_def = nullptr;   /* the captured iteration (a batch embeds it) */
     char err[512] = {0};
@@ -109,40 +111,20 @@ static void vt_ones(int K, double *vt)
         }
 }
 
-template <typename T>
-static int dalloc(admix_ctx *h, T **p, size_t count)
-{
-    const size_t b = sizeof(T) * (count ? count : 1);
-    cudaError_t e = cudaMalloc((void **)p, b);
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        return fail(h, ADMIX_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", b, cudaGetErrorString(e));
-    }
-    h->bytes += b;
-    return ADMIX_OK;
-}
-
 static void release(admix_ctx *h)
 {
     if (!h) return;
     if (h->iter_graph) cudaGraphExecDestroy(h->iter_graph);
     if (h->iter_graph_def) cudaGraphDestroy(h->iter_graph_def);
-    if (h->bed && h->owns_bed) cudaFree(h->bed);
     for (int b = 0; b < 2; ++b) {
-        if (h->sbuf[b]) cudaFree(h->sbuf[b]);
         if (h->ev_copied[b]) cudaEventDestroy(h->ev_copied[b]);
         if (h->ev_freed[b]) cudaEventDestroy(h->ev_freed[b]);
     }
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-    if (h->ll_blk) cudaFree(h->ll_blk);
     if (h->cst) { cudaStreamSynchronize(h->cst); cudaStreamDestroy(h->cst); }
     if (h->host_registered) cudaHostUnregister((void *)h->host_bed);
-    void *dps[] = {h->pkg, h->xbuf, h->parts_q, h->parts_p, h->U, h->V, h->vt, h->status_q,
-                   h->status_p, h->ll_partial, h->qn_partial, h->sc, h->counts, h->mu, h->dump};
-    for (void *p : dps)
-        if (p) cudaFree(p);
-    if (h->sc_host) cudaFreeHost(h->sc_host);
-    if (h->iter_host) cudaFreeHost(h->iter_host);
+    if (h->arena) cudaFree(h->arena);
+    if (h->dump) cudaFree(h->dump);
     if (h->st) cudaStreamDestroy(h->st);
 }
 
@@ -191,8 +173,6 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     h->I = I; h->J = J; h->K = K; h->Q = Q; h->flags = flags;
     h->Ib = (I + 3) / 4;
     h->pitch = (h->Ib + 15) / 16 * 16;
-    int rc;
-#define TRY(x) do { rc = (x); if (rc != ADMIX_OK) { strncpy(g_err, h->err, sizeof(g_err) - 1); release(h); delete h; return rc; } } while (0)
 #define TRYC(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { fail(nullptr, ADMIX_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); release(h); delete h; return ADMIX_ERR_CUDA; } } while (0)
     TRYC(cudaGetDevice(&h->dev));
     TRYC(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->dev));
@@ -215,43 +195,41 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     h->cap_spm = h->spm.S;
     h->cap_llm = h->llm.S;
 
+    Carver mem;
     if (stream_blk > 0) {
         h->streamed = true;
         h->host_bed = bed;
         h->blk = stream_blk;
         h->nblk = (int)((J + stream_blk - 1) / stream_blk);
         for (int b = 0; b < 2; ++b) {
-            TRY(dalloc(h, &h->sbuf[b], (size_t)h->pitch * stream_blk + 64));
-            TRYC(cudaMemsetAsync(h->sbuf[b], 0x55, (size_t)h->pitch * stream_blk + 64, h->st));
+            mem.add(&h->sbuf[b], (size_t)h->pitch * stream_blk + 64);
             TRYC(cudaEventCreateWithFlags(&h->ev_copied[b], cudaEventDisableTiming));
             TRYC(cudaEventCreateWithFlags(&h->ev_freed[b], cudaEventDisableTiming));
         }
         TRYC(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
         TRYC(cudaStreamCreateWithFlags(&h->cst, cudaStreamNonBlocking));
-        TRY(dalloc(h, &h->ll_blk, (size_t)h->nblk));
+        mem.add(&h->ll_blk, (size_t)h->nblk);
         cudaError_t re = cudaHostRegister((void *)bed, (size_t)h->Ib * J, cudaHostRegisterDefault);
         if (re == cudaSuccess) h->host_registered = true;
         else if (re == cudaErrorHostMemoryAlreadyRegistered) cudaGetLastError();   /* already page-locked */
         else TRYC(re);
     } else if (shared_bed) {
         h->bed = shared_bed;
-        h->owns_bed = false;
     } else {
-        TRY(dalloc(h, &h->bed, (size_t)h->pitch * J + 64));
+        mem.add(&h->bed, (size_t)h->pitch * J + 64);
     }
-    TRY(dalloc(h, &h->xbuf, (size_t)4 * nx));
-    for (int w = 0; w < 4; ++w) h->x[w] = h->xbuf + (size_t)w * nx;
-    TRY(dalloc(h, &h->parts_q, (size_t)std::max(std::max(h->sq.S, (flags & ADMIX_FLAG_MIXED) ? h->sqm.S : 1),
-                                                  h->nblk) * I * E));
-    TRY(dalloc(h, &h->parts_p, (size_t)std::max(h->sp.S, (flags & ADMIX_FLAG_MIXED) ? h->spm.S : 1) * J * E));
-    TRY(dalloc(h, &h->U, (size_t)nx * Q));
-    TRY(dalloc(h, &h->V, (size_t)nx * Q));
-    TRY(dalloc(h, &h->vt, (size_t)K * K));
-    TRY(dalloc(h, &h->status_q, (size_t)I));
+    mem.add(&h->xbuf, (size_t)4 * nx);
+    mem.add(&h->parts_q, (size_t)std::max(std::max(h->sq.S, (flags & ADMIX_FLAG_MIXED) ? h->sqm.S : 1),
+                                                  h->nblk) * I * E);
+    mem.add(&h->parts_p, (size_t)std::max(h->sp.S, (flags & ADMIX_FLAG_MIXED) ? h->spm.S : 1) * J * E);
+    mem.add(&h->U, (size_t)nx * Q);
+    mem.add(&h->V, (size_t)nx * Q);
+    mem.add(&h->vt, (size_t)K * K);
+    mem.add(&h->status_q, (size_t)I);
     if (flags & ADMIX_FLAG_MIXED)
-        TRY(dalloc(h, &h->pkg, std::max({sweep_q_mixed_pkg_bytes(K, J), sweep_p_mixed_pkg_bytes(K, I),
-                                          loglik_mixed_pkg_bytes(K, I)})));
-    TRY(dalloc(h, &h->status_p, (size_t)J));
+        mem.add(&h->pkg, std::max({sweep_q_mixed_pkg_bytes(K, J), sweep_p_mixed_pkg_bytes(K, I),
+                                          loglik_mixed_pkg_bytes(K, I)}));
+    mem.add(&h->status_p, (size_t)J);
     /* per-CTA log-likelihood partials: the resident plans, and for a streamed handle the plans of
      * a full block and of the last block (the mixed plan's count can grow as its SNP range shrinks) */
     auto ll_parts = [&](int64_t nj) {
@@ -262,18 +240,24 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     size_t n_ll = std::max((size_t)h->llp.gx, (size_t)h->llm.gx * h->llm.S);
     if (h->streamed)
         n_ll = std::max(n_ll, std::max(ll_parts(std::min<int64_t>(h->blk, J)), ll_parts(J - (int64_t)(h->nblk - 1) * h->blk)));
-    TRY(dalloc(h, &h->ll_partial, n_ll));
-    TRY(dalloc(h, &h->qn_partial, (size_t)h->qnp.blocks * (Q * Q + Q)));
-    TRY(dalloc(h, &h->sc, 1));
-    TRY(dalloc(h, &h->counts, (size_t)(I + J)));
-    TRYC(cudaMallocHost((void **)&h->sc_host, sizeof(DevScalars)));
-    TRYC(cudaMallocHost((void **)&h->iter_host, sizeof(int32_t)));
+    mem.add(&h->ll_partial, n_ll);
+    mem.add(&h->qn_partial, (size_t)h->qnp.blocks * (Q * Q + Q));
+    mem.add(&h->sc, 1);
+    mem.add(&h->counts, (size_t)(I + J));
+    if (flags & ADMIX_FLAG_MEAN_IMPUTE) mem.add(&h->mu, (size_t)J);
+    const cudaError_t ae = mem.carve(&h->arena);
+    if (ae != cudaSuccess) {
+        fail(nullptr, ADMIX_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", mem.total, cudaGetErrorString(ae));
+        release(h); delete h;
+        return ADMIX_ERR_NOMEM;
+    }
+    h->bytes += mem.total;
+    for (int w = 0; w < 4; ++w) h->x[w] = h->xbuf + (size_t)w * nx;
+    if (h->streamed)
+        for (int b = 0; b < 2; ++b) TRYC(cudaMemsetAsync(h->sbuf[b], 0x55, (size_t)h->pitch * stream_blk + 64, h->st));
 
     if (!shared_bed && !h->streamed) TRYC(upload_genotypes(h->bed, h->pitch, bed, src_pitch, I, J, on_device, h->sms, h->st));
-    if (flags & ADMIX_FLAG_MEAN_IMPUTE) {
-        TRY(dalloc(h, &h->mu, (size_t)J));
-        TRYC(launch_snp_means(h->bed, J, h->pitch, h->mu, h->st));
-    }
+    if (flags & ADMIX_FLAG_MEAN_IMPUTE) TRYC(launch_snp_means(h->bed, J, h->pitch, h->mu, h->st));
     TRYC(cudaMemsetAsync(h->xbuf, 0, sizeof(double) * 4 * nx, h->st));
     TRYC(cudaMemsetAsync(h->U, 0, sizeof(double) * nx * Q, h->st));
     TRYC(cudaMemsetAsync(h->V, 0, sizeof(double) * nx * Q, h->st));
@@ -285,7 +269,6 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     z.ll_new = NAN; z.ll_prev = NAN;
     TRYC(cudaMemcpyAsync(h->sc, &z, sizeof(z), cudaMemcpyHostToDevice, h->st));
     TRYC(cudaStreamSynchronize(h->st));
-#undef TRY
 #undef TRYC
     *out = h;
     return ADMIX_OK;
@@ -963,6 +946,7 @@ struct admix_batch {
     cudaStream_t st = nullptr;
     uint8_t *bed = nullptr;
     std::vector<admix_ctx *> m;
+    void *pinned = nullptr;          /* the members' scalar mirrors and iteration numbers */
     cudaGraphExec_t exec = nullptr;
     std::vector<int> exec_members;
     char err[512] = {0};
@@ -995,6 +979,7 @@ static void batch_release(admix_batch *b)
         delete h;
     }
     if (b->bed) cudaFree(b->bed);
+    if (b->pinned) cudaFreeHost(b->pinned);
     if (b->st) cudaStreamDestroy(b->st);
 }
 
@@ -1169,6 +1154,21 @@ static int batch_create_common(int64_t I, int64_t J, const uint8_t *bed, bool on
             bfail(nullptr, rc, "%s", msg);
             return rc;
         }
+    }
+    /* the batch graph copies the members' scalars: pinned, one block for all */
+    const size_t slot = (sizeof(DevScalars) + sizeof(int32_t) + 63) / 64 * 64;
+    e = cudaMallocHost(&b->pinned, slot * (size_t)n);
+    if (e != cudaSuccess) {
+        b->pinned = nullptr;
+        bfail(nullptr, ADMIX_ERR_CUDA, "batch scalars: %s", cudaGetErrorString(e));
+        batch_release(b); delete b;
+        return ADMIX_ERR_CUDA;
+    }
+    for (int t = 0; t < n; ++t) {
+        uint8_t *at = (uint8_t *)b->pinned + slot * (size_t)t;
+        memset(at, 0, slot);
+        b->m[t]->sc_host = (DevScalars *)at;
+        b->m[t]->iter_host = (int32_t *)(at + sizeof(DevScalars));
     }
     *out = b;
     return ADMIX_OK;

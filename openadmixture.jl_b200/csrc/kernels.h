@@ -5,10 +5,42 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
+#include <vector>
 #include "common.cuh"
 
 /* gx CTAs (= partial sums) over nunit units: nblk blocks of 128 SNPs x slices of islice individuals */
 struct LoglikPlan { int gx = 1; int64_t nblk = 1, nunit = 1, islice = 32; };
+/* Device buffers listed first, then carved from one allocation (256-byte aligned): on a B200 host an
+ * allocation takes 0.35 to 0.45 ms and its free 0.3 to 0.5, so 17 of them cost more than a small solve (and a pinned
+ * block, which single handles no longer have, 1.1 to 2.9 ms). */
+struct Carver {
+    struct Item { void **p; size_t bytes; };
+    std::vector<Item> items;
+    size_t total = 0;
+    template <typename T>
+    void add(T **p, size_t count)
+    {
+        const size_t b = (sizeof(T) * (count ? count : 1) + 255) / 256 * 256;
+        items.push_back({(void **)p, b});
+        total += b;
+    }
+    cudaError_t carve(void **arena)
+    {
+        const cudaError_t e = cudaMalloc(arena, total ? total : 256);
+        if (e != cudaSuccess) {
+            *arena = nullptr;
+            cudaGetLastError();
+            return e;
+        }
+        uint8_t *at = (uint8_t *)*arena;
+        for (const Item &i : items) {
+            *i.p = (void *)at;
+            at += i.bytes;
+        }
+        return cudaSuccess;
+    }
+};
+
 struct SweepPlan  { int gx = 1, S = 1; int64_t slice = 1; };
 
 LoglikPlan plan_loglik(int64_t I, int64_t J, int sms);

@@ -647,11 +647,10 @@ cudaError_t assign_shared_for_k(int K, const uint8_t *bed, int64_t pitch, int64_
 }
 #undef SKFR_DISPATCH
 
-template <class T>
-struct DevBuf {
-    T *p = nullptr;
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1)); }
-    ~DevBuf() { if (p) cudaFree(p); }
+/* the selection's device buffers: one allocation, freed when it ends */
+struct Arena {
+    void *p = nullptr;
+    ~Arena() { if (p) cudaFree(p); }
 };
 
 #define SK_TRY(x)                                                                                           \
@@ -673,36 +672,39 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
     const int naslice = (int)((s + SKFR_ASLICE - 1) / SKFR_ASLICE);
     const int nlists = local ? K : 1;                 /* kept lists: one for all clusters, or one per cluster */
     if ((int64_t)nslice > 65535 || (int64_t)naslice > 65535 || J > INT32_MAX) return cudaErrorInvalidValue;
-    DevBuf<int64_t> d_cnt;
-    DevBuf<double> d_xt, d_ab, d_sq, d_partial, d_D, d_theta, d_score, d_pt, d_apart, d_sc;
-    DevBuf<uint32_t> d_mask;
-    DevBuf<int32_t> d_cl, d_cl2, d_nk, d_changed, d_S, d_M, d_kept;
-    SK_TRY(d_cnt.alloc(3 * J));
-    SK_TRY(d_xt.alloc(4 * J));
-    SK_TRY(d_ab.alloc(2 * J));
-    SK_TRY(d_sq.alloc(4 * J));
-    SK_TRY(d_partial.alloc((size_t)nslice * I));
-    SK_TRY(d_D.alloc(I));
-    SK_TRY(d_theta.alloc((size_t)K * J));
-    SK_TRY(d_score.alloc((size_t)nlists * J));
+    int64_t *d_cnt;
+    double *d_xt, *d_ab, *d_sq, *d_partial, *d_D, *d_theta, *d_score, *d_pt, *d_apart, *d_sc;
+    uint32_t *d_mask;
+    int32_t *d_cl, *d_cl2, *d_nk, *d_changed, *d_S, *d_M, *d_kept;
     const int64_t npair = (s + 1) / 2;                /* kept-list pairs */
-    SK_TRY(d_pt.alloc((size_t)K * npair * 16));
-    SK_TRY(d_apart.alloc((size_t)naslice * I * K));
-    SK_TRY(d_sc.alloc((size_t)I * K));
-    SK_TRY(d_mask.alloc((size_t)K * nw));
-    SK_TRY(d_cl.alloc(I));
-    SK_TRY(d_cl2.alloc(I));
-    SK_TRY(d_nk.alloc(K));
-    SK_TRY(d_changed.alloc(1));
-    SK_TRY(d_S.alloc((size_t)K * J));
-    SK_TRY(d_M.alloc((size_t)K * J));
-    SK_TRY(d_kept.alloc((size_t)nlists * s));
+    Carver mem;
+    mem.add(&d_cnt, (size_t)(3 * J));
+    mem.add(&d_xt, (size_t)(4 * J));
+    mem.add(&d_ab, (size_t)(2 * J));
+    mem.add(&d_sq, (size_t)(4 * J));
+    mem.add(&d_partial, (size_t)(nslice * I));
+    mem.add(&d_D, (size_t)(I));
+    mem.add(&d_theta, (size_t)(K * J));
+    mem.add(&d_score, (size_t)(nlists * J));
+    mem.add(&d_pt, (size_t)(K * npair * 16));
+    mem.add(&d_apart, (size_t)(naslice * I * K));
+    mem.add(&d_sc, (size_t)(I * K));
+    mem.add(&d_mask, (size_t)(K * nw));
+    mem.add(&d_cl, (size_t)(I));
+    mem.add(&d_cl2, (size_t)(I));
+    mem.add(&d_nk, (size_t)(K));
+    mem.add(&d_changed, (size_t)(1));
+    mem.add(&d_S, (size_t)(K * J));
+    mem.add(&d_M, (size_t)(K * J));
+    mem.add(&d_kept, (size_t)(nlists * s));
+    Arena arena;
+    SK_TRY(mem.carve(&arena.p));
 
     /* per-SNP standardisation from the class counts (host FP64, as the oracle) */
-    k_skfr_counts<<<(unsigned)((J + 3) / 4), 128, 0, st>>>(bed, pitch, nw, J, d_cnt.p);
+    k_skfr_counts<<<(unsigned)((J + 3) / 4), 128, 0, st>>>(bed, pitch, nw, J, d_cnt);
     SK_TRY(cudaGetLastError());
     std::vector<int64_t> cnt((size_t)3 * J);
-    SK_TRY(cudaMemcpyAsync(cnt.data(), d_cnt.p, sizeof(int64_t) * 3 * J, cudaMemcpyDeviceToHost, st));
+    SK_TRY(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int64_t) * 3 * J, cudaMemcpyDeviceToHost, st));
     SK_TRY(cudaStreamSynchronize(st));
     std::vector<double> xt((size_t)4 * J), ab((size_t)2 * J);
     double x2_total = 0.0;
@@ -726,8 +728,8 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
         xt[4 * l + 2] = a - b;
         xt[4 * l + 3] = 2.0 * a - b;
     }
-    SK_TRY(cudaMemcpyAsync(d_xt.p, xt.data(), sizeof(double) * 4 * J, cudaMemcpyHostToDevice, st));
-    SK_TRY(cudaMemcpyAsync(d_ab.p, ab.data(), sizeof(double) * 2 * J, cudaMemcpyHostToDevice, st));
+    SK_TRY(cudaMemcpyAsync(d_xt, xt.data(), sizeof(double) * 4 * J, cudaMemcpyHostToDevice, st));
+    SK_TRY(cudaMemcpyAsync(d_ab, ab.data(), sizeof(double) * 2 * J, cudaMemcpyHostToDevice, st));
 
     SplitMix64 rng{seed};
     std::vector<double> D((size_t)I), dk((size_t)I * K), sc((size_t)I * K);
@@ -737,38 +739,38 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
 
     /* squared distances of every individual to individual `center` over all SNPs, into out (host) */
     auto dist = [&](int64_t center, double *out) -> cudaError_t {
-        k_skfr_sqtab<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(bed, pitch, J, d_xt.p, center, d_sq.p);
+        k_skfr_sqtab<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(bed, pitch, J, d_xt, center, d_sq);
         SK_TRY(cudaGetLastError());
         const dim3 grid((unsigned)((nw + 127) / 128), (unsigned)nslice);
-        k_skfr_dist<<<grid, 128, 0, st>>>(bed, pitch, I, J, d_sq.p, d_partial.p);
+        k_skfr_dist<<<grid, 128, 0, st>>>(bed, pitch, I, J, d_sq, d_partial);
         SK_TRY(cudaGetLastError());
-        k_skfr_dist_sum<<<(unsigned)((I + 255) / 256), 256, 0, st>>>(d_partial.p, I, nslice, d_D.p);
+        k_skfr_dist_sum<<<(unsigned)((I + 255) / 256), 256, 0, st>>>(d_partial, I, nslice, d_D);
         SK_TRY(cudaGetLastError());
-        SK_TRY(cudaMemcpyAsync(out, d_D.p, sizeof(double) * I, cudaMemcpyDeviceToHost, st));
+        SK_TRY(cudaMemcpyAsync(out, d_D, sizeof(double) * I, cudaMemcpyDeviceToHost, st));
         return cudaStreamSynchronize(st);
     };
     /* for the assignment dcl: cluster sizes, centres, scores, kept lists, pair tables and sc[i][k] (no sync) */
     auto pass = [&](const int32_t *dcl) -> cudaError_t {
-        SK_TRY(cudaMemsetAsync(d_nk.p, 0, sizeof(int32_t) * K, st));
-        k_skfr_masks<<<(unsigned)((nw + 127) / 128), 128, 0, st>>>(dcl, I, nw, K, d_mask.p, d_nk.p);
+        SK_TRY(cudaMemsetAsync(d_nk, 0, sizeof(int32_t) * K, st));
+        k_skfr_masks<<<(unsigned)((nw + 127) / 128), 128, 0, st>>>(dcl, I, nw, K, d_mask, d_nk);
         SK_TRY(cudaGetLastError());
-        SK_TRY(sums_for_k(K, bed, pitch, nw, J, d_mask.p, d_S.p, d_M.p, st));
-        k_skfr_means<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(d_S.p, d_M.p, d_cnt.p, I, d_ab.p, d_nk.p, K, J, local,
-                                                                d_theta.p, d_score.p);
+        SK_TRY(sums_for_k(K, bed, pitch, nw, J, d_mask, d_S, d_M, st));
+        k_skfr_means<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(d_S, d_M, d_cnt, I, d_ab, d_nk, K, J, local,
+                                                                d_theta, d_score);
         SK_TRY(cudaGetLastError());
-        k_skfr_select<<<(unsigned)nlists, SKFR_SEL_THREADS, 0, st>>>(d_score.p, J, s, d_kept.p);
+        k_skfr_select<<<(unsigned)nlists, SKFR_SEL_THREADS, 0, st>>>(d_score, J, s, d_kept);
         SK_TRY(cudaGetLastError());
-        k_skfr_pairs<<<(unsigned)((K * npair + 255) / 256), 256, 0, st>>>(d_theta.p, d_xt.p, d_kept.p, s, local ? s : 0, K,
-                                                                         J, d_pt.p);
+        k_skfr_pairs<<<(unsigned)((K * npair + 255) / 256), 256, 0, st>>>(d_theta, d_xt, d_kept, s, local ? s : 0, K,
+                                                                         J, d_pt);
         SK_TRY(cudaGetLastError());
         if (local) {
             const dim3 grid((unsigned)((I + 127) / 128), (unsigned)naslice, (unsigned)K);
-            k_skfr_assign_own<<<grid, 128, 0, st>>>(bed, pitch, I, d_kept.p, s, K, d_pt.p, d_apart.p);
+            k_skfr_assign_own<<<grid, 128, 0, st>>>(bed, pitch, I, d_kept, s, K, d_pt, d_apart);
             SK_TRY(cudaGetLastError());
         } else {
-            SK_TRY(assign_shared_for_k(K, bed, pitch, I, d_kept.p, s, d_pt.p, d_apart.p, st));
+            SK_TRY(assign_shared_for_k(K, bed, pitch, I, d_kept, s, d_pt, d_apart, st));
         }
-        k_skfr_assign_sum<<<(unsigned)((I * K + 255) / 256), 256, 0, st>>>(d_apart.p, I * K, naslice, d_sc.p);
+        k_skfr_assign_sum<<<(unsigned)((I * K + 255) / 256), 256, 0, st>>>(d_apart, I * K, naslice, d_sc);
         return cudaGetLastError();
     };
 
@@ -801,18 +803,18 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
                 if (dk[(size_t)k * I + i] < dk[(size_t)best * I + i]) best = k;
             cl[i] = best;
         }
-        int32_t *cur = d_cl.p, *nxt = d_cl2.p;
+        int32_t *cur = d_cl, *nxt = d_cl2;
         SK_TRY(cudaMemcpyAsync(cur, cl.data(), sizeof(int32_t) * I, cudaMemcpyHostToDevice, st));
         /* iterations: the host reads one count per iteration */
         int it = 0;
         bool converged = false;
         for (it = 1; it <= max_iter; ++it) {
             SK_TRY(pass(cur));
-            SK_TRY(cudaMemsetAsync(d_changed.p, 0, sizeof(int32_t), st));
-            k_skfr_argmin<<<(unsigned)((I + 255) / 256), 256, 0, st>>>(d_sc.p, I, K, cur, nxt, d_changed.p);
+            SK_TRY(cudaMemsetAsync(d_changed, 0, sizeof(int32_t), st));
+            k_skfr_argmin<<<(unsigned)((I + 255) / 256), 256, 0, st>>>(d_sc, I, K, cur, nxt, d_changed);
             SK_TRY(cudaGetLastError());
             int32_t changed = 0;
-            SK_TRY(cudaMemcpyAsync(&changed, d_changed.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+            SK_TRY(cudaMemcpyAsync(&changed, d_changed, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
             SK_TRY(cudaStreamSynchronize(st));
             if (changed == 0) {
                 converged = true;
@@ -824,9 +826,9 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
         /* the objective of the final assignment with its sparse centres: at convergence the last pass
          * was already of this assignment */
         if (!converged) SK_TRY(pass(cur));
-        SK_TRY(cudaMemcpyAsync(sc.data(), d_sc.p, sizeof(double) * I * K, cudaMemcpyDeviceToHost, st));
+        SK_TRY(cudaMemcpyAsync(sc.data(), d_sc, sizeof(double) * I * K, cudaMemcpyDeviceToHost, st));
         SK_TRY(cudaMemcpyAsync(cl.data(), cur, sizeof(int32_t) * I, cudaMemcpyDeviceToHost, st));
-        SK_TRY(cudaMemcpyAsync(kept.data(), d_kept.p, sizeof(int32_t) * nlists * s, cudaMemcpyDeviceToHost, st));
+        SK_TRY(cudaMemcpyAsync(kept.data(), d_kept, sizeof(int32_t) * nlists * s, cudaMemcpyDeviceToHost, st));
         SK_TRY(cudaStreamSynchronize(st));
         double obj = x2_total;
         for (int64_t i = 0; i < I; ++i) obj += sc[(size_t)i * K + cl[i]];
