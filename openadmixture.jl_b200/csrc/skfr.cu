@@ -7,9 +7,9 @@
  * pinned exactly by the CPU oracle (oracle/skfr_oracle.py), whose header states them.
  *
  * Device work, all on the handle's padded genotypes (padding coded missing):
- *   - per-SNP class counts by popcount of the code bit planes (k_skfr_counts);
+ *   - per-SNP class counts by popcount of the code bit planes and the standardisation (k_skfr_stats);
  *   - k-means++ seeding distances ||x_i - x_c||^2 over all SNPs: the squared difference of every
- *     (SNP, code) to the centre in a table (k_skfr_sqtab), then a thread owns 16 individuals (one
+ *     (SNP, code) to the centre in a table (k_skfr_sqtab), then a thread owns 8 individuals (half a
  *     32-bit word of a column) and a slice of SKFR_SLICE SNPs, adding table entries staged in
  *     shared memory in FP64, the slice sums added in slice order (k_skfr_dist, k_skfr_dist_sum);
  *   - per iteration, the cluster sums of every SNP as exact integers: membership bit masks per
@@ -19,7 +19,7 @@
  *     memory); the last cluster's sums are the SNP's totals less the others'; centres and feature
  *     scores in FP64 (k_skfr_means);
  *   - the `sparsity` largest scores of each kept list (ties to the lower index) by a radix select
- *     on the scores' bit patterns and an index-order compaction, one block per list (k_skfr_select);
+ *     on the scores' bit patterns and an index-order compaction, one cluster of blocks per list (k_skfr_select);
  *   - the reassignment scores of every individual on the kept SNPs: the terms of each two
  *     consecutive kept SNPs added for all 16 code pairs (k_skfr_pairs), then one thread per
  *     individual and slice of SKFR_ASLICE kept SNPs adds one pair entry per two SNPs in FP64, in SNP
@@ -33,6 +33,7 @@
  * round-to-nearest intrinsics, so no multiply-add is contracted.
  */
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -47,15 +48,21 @@ constexpr int SKFR_WCHUNK = 256;     /* 16-individual words of masks staged per 
 constexpr int SKFR_ASLICE = 1024;    /* kept SNPs per partial sum of the reassignment scores */
 constexpr int SKFR_ACHUNK = 32;      /* kept SNPs whose pair tables are staged in shared memory at a time */
 constexpr int SKFR_SEL_THREADS = 1024;
+constexpr int SKFR_SEL_CTAS = 8;     /* blocks of a list's cluster */
 
 __device__ __forceinline__ uint32_t col_word(const uint8_t *bed, int64_t pitch, int64_t l, int64_t w)
 {
     return *(const uint32_t *)(bed + (size_t)l * pitch + (size_t)w * 4);
 }
 
-/* class counts of every SNP: n0 (code 00, dosage 0), n1 (10, dosage 1), n2 (11, dosage 2) */
-__global__ void k_skfr_counts(const uint8_t *__restrict__ bed, int64_t pitch, int64_t nw, int64_t J,
-                              int64_t *__restrict__ cnt)
+/* Class counts of every SNP, n0 (code 00, dosage 0), n1 (10, dosage 1), n2 (11, dosage 2), and its standardisation:
+ * a = 1 / sigma, b = mu / sigma (0 where monomorphic or without genotypes), the values xt[code] of the four
+ * codes, and the sum over the polymorphic SNPs of their non-missing counts (exact integers).  One warp per SNP;
+ * the arithmetic is the oracle's, operation by operation.  On the host this took a copy of the counts, a loop over
+ * the SNPs and a copy back (7 MB over the bus at J=100k, with the device idle); the kernel takes 0.09 ms. */
+__global__ void k_skfr_stats(const uint8_t *__restrict__ bed, int64_t pitch, int64_t nw, int64_t J,
+                             int64_t *__restrict__ cnt, double *__restrict__ xt, double *__restrict__ ab,
+                             unsigned long long *__restrict__ x2)
 {
     const int64_t l = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
@@ -77,6 +84,23 @@ __global__ void k_skfr_counts(const uint8_t *__restrict__ bed, int64_t pitch, in
         cnt[3 * l] = c0;
         cnt[3 * l + 1] = c1;
         cnt[3 * l + 2] = c2;
+        const double n1 = (double)c1, n2 = (double)c2, n = (double)(c0 + c1 + c2);
+        double a = 0.0, b = 0.0;
+        if (n > 0.0) {
+            const double mu = __ddiv_rn(__dadd_rn(n1, __dmul_rn(2.0, n2)), n);
+            const double var = __dsub_rn(__ddiv_rn(__dadd_rn(n1, __dmul_rn(4.0, n2)), n), __dmul_rn(mu, mu));
+            if (var > 0.0) {
+                a = __ddiv_rn(1.0, __dsqrt_rn(var));
+                b = __dmul_rn(mu, a);
+                atomicAdd(x2, (unsigned long long)(c0 + c1 + c2));
+            }
+        }
+        ab[2 * l] = a;
+        ab[2 * l + 1] = b;
+        xt[4 * l] = -b;
+        xt[4 * l + 1] = 0.0;
+        xt[4 * l + 2] = __dsub_rn(a, b);
+        xt[4 * l + 3] = __dsub_rn(__dmul_rn(2.0, a), b);
     }
 }
 
@@ -95,50 +119,53 @@ __global__ void k_skfr_sqtab(const uint8_t *__restrict__ bed, int64_t pitch, int
     }
 }
 
-/* partial[s][i] = sum over the SNPs l of slice s, in order, of sq[l][code_il] */
+/* partial[s][i] = sum over the SNPs l of slice s, in order, of sq[l][code_il].  A thread owns 8 individuals (a
+ * half-word of a column): the adds of one individual are a serial chain, so the threads are what fills the SMs (16 a
+ * thread left 13 warps per SM at I=10k, J=100k: 429 us per centre, now 307).  Bound: one shared 8-byte load per cell. */
 __global__ void __launch_bounds__(128)
 k_skfr_dist(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, int64_t J, const double *__restrict__ sq,
             double *__restrict__ partial)
 {
-    __shared__ double tab[SKFR_DCHUNK * 4];
-    const int64_t w = (int64_t)blockIdx.x * 128 + threadIdx.x;   /* word = 16 individuals */
+    constexpr int NP = 8;
+    __shared__ __align__(16) double tab[SKFR_DCHUNK * 4];
+    const int64_t w = (int64_t)blockIdx.x * 128 + threadIdx.x;   /* 8 individuals */
     const int64_t s = blockIdx.y;
-    const bool live = w * 16 < I;
+    const bool live = w * NP < I;
     const int64_t l0 = s * SKFR_SLICE, l1 = min(J, l0 + SKFR_SLICE);
-    double part[16];
+    double part[NP];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) part[j] = 0.0;
+    for (int j = 0; j < NP; ++j) part[j] = 0.0;
     for (int64_t c0 = l0; c0 < l1; c0 += SKFR_DCHUNK) {
         const int n = (int)min((int64_t)SKFR_DCHUNK, l1 - c0);
         __syncthreads();
-        for (int t = threadIdx.x; t < 4 * n; t += 128) tab[t] = sq[4 * c0 + t];
+        for (int t = threadIdx.x; t < 2 * n; t += 128) ((double2 *)tab)[t] = ((const double2 *)(sq + 4 * c0))[t];
         __syncthreads();
         if (live) {
-            const uint8_t *col = bed + (size_t)c0 * pitch + (size_t)w * 4;
+            const uint8_t *col = bed + (size_t)c0 * pitch + (size_t)w * 2;
             int u = 0;
-            for (; u + 4 <= n; u += 4) {
-                uint32_t x[4];
+            for (; u + 8 <= n; u += 8) {
+                uint32_t x[8];
 #pragma unroll
-                for (int v = 0; v < 4; ++v) x[v] = *(const uint32_t *)(col + (size_t)(u + v) * pitch);
+                for (int v = 0; v < 8; ++v) x[v] = *(const uint16_t *)(col + (size_t)(u + v) * pitch);
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
+                for (int v = 0; v < 8; ++v) {
                     const double *tb = tab + (u + v) * 4;
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) part[j] = __dadd_rn(part[j], tb[(x[v] >> (2 * j)) & 3u]);
+                    for (int j = 0; j < NP; ++j) part[j] = __dadd_rn(part[j], tb[(x[v] >> (2 * j)) & 3u]);
                 }
             }
             for (; u < n; ++u) {
-                const uint32_t x = *(const uint32_t *)(col + (size_t)u * pitch);
+                const uint32_t x = *(const uint16_t *)(col + (size_t)u * pitch);
                 const double *tb = tab + u * 4;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) part[j] = __dadd_rn(part[j], tb[(x >> (2 * j)) & 3u]);
+                for (int j = 0; j < NP; ++j) part[j] = __dadd_rn(part[j], tb[(x >> (2 * j)) & 3u]);
             }
         }
     }
     if (live) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (w * 16 + j < I) partial[(size_t)s * I + w * 16 + j] = part[j];
+        for (int j = 0; j < NP; ++j)
+            if (w * NP + j < I) partial[(size_t)s * I + w * NP + j] = part[j];
     }
 }
 
@@ -326,68 +353,125 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *wsum, 
     return before;
 }
 
-/* The s largest of the J scores of list blockIdx.x (ties to the lower index), written to out in
+/* Suffix counts of a 256-bin histogram over threads 0..255 (bin tid): *bin = the largest b whose bins >= b hold at
+ * least `rank` entries, *left = rank less the entries of the bins above b. */
+__device__ __forceinline__ void pick_bin(uint32_t n, long long rank, uint32_t *wsum, int *bin, long long *left)
+{
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    uint32_t x = n;                                   /* this bin and those above it in the warp */
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_down_sync(0xffffffffu, x, o);
+        if (lane + o < 32) x += y;
+    }
+    if (tid < 256 && lane == 0) wsum[wid] = x;
+    __syncthreads();
+    if (tid < 256) {
+        for (int w = wid + 1; w < 8; ++w) x += wsum[w];
+        const long long here = x, above = (long long)x - n;
+        if (here >= rank && above < rank) {
+            *bin = tid;
+            *left = rank - above;
+        }
+    }
+    __syncthreads();
+}
+
+/* The s largest of the J scores of one list (ties to the lower index), written to out in
  * increasing index order.  The scores are non-negative doubles, so their bit patterns order as the
  * values: eight radix passes of 8 bits find the s-th largest pattern T and how many copies of it
  * are needed; one pass in index order then keeps every score above T and the first `need` equal
  * to T, each thread taking 4 consecutive SNPs and one packed scan of (above, equal) counts giving
- * every kept SNP its output position. */
-__global__ void __launch_bounds__(SKFR_SEL_THREADS)
+ * every kept SNP its output position.
+ * A cluster of SKFR_SEL_CTAS blocks per list, each owning a range of SNPs, adds its histograms and
+ * counts through distributed shared memory: one block alone was bound by the latency of its own passes
+ * over the list (J=100k: 271 us, 52 us with 8). */
+__global__ void __cluster_dims__(SKFR_SEL_CTAS, 1, 1) __launch_bounds__(SKFR_SEL_THREADS)
 k_skfr_select(const double *__restrict__ score, int64_t J, int64_t s, int32_t *__restrict__ out)
 {
-    __shared__ uint32_t hist[256];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ uint32_t hist[2][256];
     __shared__ uint32_t wsum[32];
-    __shared__ unsigned long long s_prefix;
+    __shared__ unsigned long long cnt[2];             /* this block's scores above T and equal to it */
+    __shared__ int s_bin;
     __shared__ long long s_rank;
-    const unsigned long long *key = (const unsigned long long *)(score + (size_t)blockIdx.x * J);
-    int32_t *o = out + (size_t)blockIdx.x * s;
+    const int list = blockIdx.x / SKFR_SEL_CTAS, rank_c = (int)cl.block_rank();
+    const unsigned long long *key = (const unsigned long long *)(score + (size_t)list * J);
+    int32_t *o = out + (size_t)list * s;
     const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t per = ((J + SKFR_SEL_CTAS - 1) / SKFR_SEL_CTAS + 3) / 4 * 4;
+    const int64_t la = min(J, per * rank_c), lz = min(J, la + per);
+    if (tid < 256) hist[0][tid] = 0u;
+    __syncthreads();
     unsigned long long prefix = 0ull, pmask = 0ull;
     long long rank = s;                     /* rank of the wanted pattern among those under the prefix */
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        for (int t = tid; t < 256; t += SKFR_SEL_THREADS) hist[t] = 0u;
-        __syncthreads();
-        for (int64_t l0 = 0; l0 < J; l0 += 4 * SKFR_SEL_THREADS) {
+    for (int pass = 0; pass < 8; ++pass) {
+        const int shift = 56 - 8 * pass;
+        uint32_t *h = hist[pass & 1];
+        for (int64_t l0 = la; l0 < lz; l0 += 4 * SKFR_SEL_THREADS) {
             unsigned long long kv[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 const int64_t l = l0 + tid + (int64_t)v * SKFR_SEL_THREADS;
-                kv[v] = l < J ? key[l] : 0ull;
+                kv[v] = l < lz ? key[l] : 0ull;
             }
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 const int64_t l = l0 + tid + (int64_t)v * SKFR_SEL_THREADS;
-                const bool act = l < J && (kv[v] & pmask) == prefix;
+                const bool act = l < lz && (kv[v] & pmask) == prefix;
+                if (!__any_sync(0xffffffffu, act)) continue;
                 const uint32_t bin = act ? (uint32_t)((kv[v] >> shift) & 255u) : 256u;
                 const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-                if (act && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
+                if (act && lane == __ffs(peers) - 1) atomicAdd(&h[bin], (uint32_t)__popc(peers));
             }
         }
-        __syncthreads();
-        if (tid == 0) {
-            long long acc = 0;
-            int b = 255;
-            for (; b > 0; --b) {
-                if (acc + (long long)hist[b] >= rank) break;
-                acc += hist[b];
-            }
-            s_prefix = prefix | ((unsigned long long)b << shift);
-            s_rank = rank - acc;
+        /* every block's counts are in; the other buffer is free (its readers passed this barrier after reading it) */
+        cl.sync();
+        uint32_t n = 0;
+        if (tid < 256) {
+            for (int b = 0; b < SKFR_SEL_CTAS; ++b) n += cl.map_shared_rank(h, b)[tid];
+            hist[(pass + 1) & 1][tid] = 0u;
         }
-        __syncthreads();
-        prefix = s_prefix;
+        pick_bin(n, rank, wsum, &s_bin, &s_rank);
+        prefix |= (unsigned long long)s_bin << shift;
         rank = s_rank;
         pmask |= 255ull << shift;
+        __syncthreads();                              /* s_bin and s_rank are read */
     }
     const unsigned long long T = prefix;
     const uint32_t need = (uint32_t)rank;   /* copies of T kept; s - need patterns lie above T */
-    uint32_t base_gt = 0, base_eq = 0;
-    for (int64_t l0 = 0; l0 < J; l0 += 4 * SKFR_SEL_THREADS) {
+    uint32_t gt0 = 0, eq0 = 0;
+    for (int64_t l = la + tid; l < lz; l += SKFR_SEL_THREADS) {
+        const unsigned long long kv = key[l];
+        gt0 += kv > T;
+        eq0 += kv == T;
+    }
+    if (tid < 2) cnt[tid] = 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        gt0 += __shfl_down_sync(0xffffffffu, gt0, w);
+        eq0 += __shfl_down_sync(0xffffffffu, eq0, w);
+    }
+    if (lane == 0) {
+        if (gt0) atomicAdd(&cnt[0], (unsigned long long)gt0);
+        if (eq0) atomicAdd(&cnt[1], (unsigned long long)eq0);
+    }
+    cl.sync();
+    uint32_t base_gt = 0, base_eq = 0;                /* of the blocks before this one */
+    for (int b = 0; b < rank_c; ++b) {
+        const unsigned long long *c = cl.map_shared_rank(cnt, b);
+        base_gt += (uint32_t)c[0];
+        base_eq += (uint32_t)c[1];
+    }
+    cl.sync();                                        /* nobody leaves while its counts are read */
+    for (int64_t l0 = la; l0 < lz; l0 += 4 * SKFR_SEL_THREADS) {
         const int64_t lb = l0 + 4 * (int64_t)tid;
         uint32_t gt = 0, eq = 0, gtm = 0, eqm = 0;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            if (lb + v < J) {
+            if (lb + v < lz) {
                 const unsigned long long kv = key[lb + v];
                 if (kv > T) { gt++; gtm |= 1u << v; }
                 else if (kv == T) { eq++; eqm |= 1u << v; }
@@ -414,10 +498,12 @@ k_skfr_select(const double *__restrict__ score, int64_t J, int64_t s, int32_t *_
 /* Pair tables of the reassignment terms.  For cluster k and pair r of its kept list (list k * kstride:
  * one shared list when kstride is 0; list positions q = 2r and q + 1) and codes c1, c2:
  * pt[k][r][4 c1 + c2] = T(q, c1) + T(q + 1, c2), with T(p, c) = theta_kl^2 - (2 x_l,c) theta_kl for l
- * the SNP at position p; an odd last position alone gives T(q, c1) for every c2. */
+ * the SNP at position p; an odd last position alone gives T(q, c1) for every c2.  With one shared list (kstride 0)
+ * the tables are laid out as the reassignment stages them: pt[r][4 c1 + c2][k], K | 1 doubles a row. */
 __global__ void k_skfr_pairs(const double *__restrict__ theta, const double *__restrict__ xt, const int32_t *__restrict__ kept,
                              int64_t nkept, int64_t kstride, int K, int64_t J, double *__restrict__ pt)
 {
+    const int KS = K | 1;                             /* one shared list: [pair][code pair][k], row stride KS */
     const int64_t npair = (nkept + 1) / 2;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (int64_t)K * npair) return;
@@ -438,11 +524,12 @@ __global__ void k_skfr_pairs(const double *__restrict__ theta, const double *__r
 #pragma unroll
         for (int c = 0; c < 4; ++c) b[c] = __dsub_rn(tt, __dmul_rn(__dmul_rn(2.0, xt[4 * l + c]), th));
     }
-    double *o = pt + (size_t)t * 16;
+    double *o = kstride ? pt + (size_t)t * 16 : pt + (size_t)r * 16 * KS + k;
+    const int os = kstride ? 1 : KS;
 #pragma unroll
     for (int c1 = 0; c1 < 4; ++c1)
 #pragma unroll
-        for (int c2 = 0; c2 < 4; ++c2) o[4 * c1 + c2] = two ? __dadd_rn(a[c1], b[c2]) : a[c1];
+        for (int c2 = 0; c2 < 4; ++c2) o[(4 * c1 + c2) * os] = two ? __dadd_rn(a[c1], b[c2]) : a[c1];
 }
 
 /* The codes of a chunk's kept SNPs for a block's 128 individuals (32 bytes per SNP): thread t loads
@@ -475,16 +562,16 @@ __device__ __forceinline__ void store_codes(uint8_t (*cp)[64], uint2 v)
  * tables as [pair][code pair][k] with an odd row stride (the 16 code pairs of one pair fall in
  * different banks) and the chunk's codes interleaved by pair (one 16-bit load per pair and thread),
  * the codes of the next chunk loaded while this one is summed; each code is read once for all K
- * clusters. */
+ * clusters.  The tables arrive in the staged layout: regrouping them here took a division per element,
+ * more instructions than the sums (I=10k, 10k kept of J=100k, K=5: 187 us, now 106). */
 template <int K>
 __global__ void __launch_bounds__(128)
 k_skfr_assign_shared(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, const int32_t *__restrict__ kept,
                      int64_t nkept, const double *__restrict__ pt, double *__restrict__ part)
 {
     constexpr int KS = K | 1;
-    __shared__ double ts[(SKFR_ACHUNK / 2) * 16 * KS];
+    __shared__ __align__(16) double ts[(SKFR_ACHUNK / 2) * 16 * KS];
     __shared__ __align__(16) uint8_t cp[SKFR_ACHUNK / 2][64];
-    const int64_t npair = (nkept + 1) / 2;
     const int64_t i0 = (int64_t)blockIdx.x * 128, i = i0 + threadIdx.x;
     const int64_t p0 = (int64_t)blockIdx.y * SKFR_ASLICE, p1 = min(nkept, p0 + SKFR_ASLICE);
     const int sh = (int)(threadIdx.x & 3) * 2, cb = 2 * (int)(threadIdx.x >> 2);
@@ -496,9 +583,9 @@ k_skfr_assign_shared(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, 
         const int n = (int)min((int64_t)SKFR_ACHUNK, p1 - q0), np = (n + 1) / 2;
         const int64_t r0 = q0 / 2;
         __syncthreads();
-        for (int t = threadIdx.x; t < np * 16 * K; t += 128) {
-            const int k = t / (np * 16), e = t - k * (np * 16);       /* e = pair * 16 + code pair */
-            ts[e * KS + k] = pt[((size_t)k * npair + r0) * 16 + e];
+        {   /* np * 16 rows of KS doubles, contiguous: 16 KS doubles a pair, so whole 16-byte groups */
+            const double2 *src = (const double2 *)(pt + (size_t)r0 * 16 * KS);
+            for (int t = threadIdx.x; t < np * 8 * KS; t += 128) ((double2 *)ts)[t] = src[t];
         }
         store_codes(cp, cv);
         if (q0 + SKFR_ACHUNK < p1)
@@ -673,12 +760,14 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
     const int nlists = local ? K : 1;                 /* kept lists: one for all clusters, or one per cluster */
     if ((int64_t)nslice > 65535 || (int64_t)naslice > 65535 || J > INT32_MAX) return cudaErrorInvalidValue;
     int64_t *d_cnt;
+    unsigned long long *d_x2;
     double *d_xt, *d_ab, *d_sq, *d_partial, *d_D, *d_theta, *d_score, *d_pt, *d_apart, *d_sc;
     uint32_t *d_mask;
     int32_t *d_cl, *d_cl2, *d_nk, *d_changed, *d_S, *d_M, *d_kept;
     const int64_t npair = (s + 1) / 2;                /* kept-list pairs */
     Carver mem;
     mem.add(&d_cnt, (size_t)(3 * J));
+    mem.add(&d_x2, 1);
     mem.add(&d_xt, (size_t)(4 * J));
     mem.add(&d_ab, (size_t)(2 * J));
     mem.add(&d_sq, (size_t)(4 * J));
@@ -686,7 +775,7 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
     mem.add(&d_D, (size_t)(I));
     mem.add(&d_theta, (size_t)(K * J));
     mem.add(&d_score, (size_t)(nlists * J));
-    mem.add(&d_pt, (size_t)(K * npair * 16));
+    mem.add(&d_pt, (size_t)((K | 1) * npair * 16));
     mem.add(&d_apart, (size_t)(naslice * I * K));
     mem.add(&d_sc, (size_t)(I * K));
     mem.add(&d_mask, (size_t)(K * nw));
@@ -700,36 +789,13 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
     Arena arena;
     SK_TRY(mem.carve(&arena.p));
 
-    /* per-SNP standardisation from the class counts (host FP64, as the oracle) */
-    k_skfr_counts<<<(unsigned)((J + 3) / 4), 128, 0, st>>>(bed, pitch, nw, J, d_cnt);
+    SK_TRY(cudaMemsetAsync(d_x2, 0, sizeof(unsigned long long), st));
+    k_skfr_stats<<<(unsigned)((J + 3) / 4), 128, 0, st>>>(bed, pitch, nw, J, d_cnt, d_xt, d_ab, d_x2);
     SK_TRY(cudaGetLastError());
-    std::vector<int64_t> cnt((size_t)3 * J);
-    SK_TRY(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int64_t) * 3 * J, cudaMemcpyDeviceToHost, st));
+    unsigned long long x2 = 0;
+    SK_TRY(cudaMemcpyAsync(&x2, d_x2, sizeof(x2), cudaMemcpyDeviceToHost, st));
     SK_TRY(cudaStreamSynchronize(st));
-    std::vector<double> xt((size_t)4 * J), ab((size_t)2 * J);
-    double x2_total = 0.0;
-    for (int64_t l = 0; l < J; ++l) {
-        const double n0 = (double)cnt[3 * l], n1 = (double)cnt[3 * l + 1], n2 = (double)cnt[3 * l + 2];
-        const double n = n0 + n1 + n2;
-        double a = 0.0, b = 0.0;
-        if (n > 0.0) {
-            const double mu = (n1 + 2.0 * n2) / n;
-            const double var = (n1 + 4.0 * n2) / n - mu * mu;
-            if (var > 0.0) {
-                a = 1.0 / sqrt(var);
-                b = mu * a;
-                x2_total += n;
-            }
-        }
-        ab[2 * l] = a;
-        ab[2 * l + 1] = b;
-        xt[4 * l] = -b;
-        xt[4 * l + 1] = 0.0;
-        xt[4 * l + 2] = a - b;
-        xt[4 * l + 3] = 2.0 * a - b;
-    }
-    SK_TRY(cudaMemcpyAsync(d_xt, xt.data(), sizeof(double) * 4 * J, cudaMemcpyHostToDevice, st));
-    SK_TRY(cudaMemcpyAsync(d_ab, ab.data(), sizeof(double) * 2 * J, cudaMemcpyHostToDevice, st));
+    const double x2_total = (double)x2;
 
     SplitMix64 rng{seed};
     std::vector<double> D((size_t)I), dk((size_t)I * K), sc((size_t)I * K);
@@ -741,7 +807,7 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
     auto dist = [&](int64_t center, double *out) -> cudaError_t {
         k_skfr_sqtab<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(bed, pitch, J, d_xt, center, d_sq);
         SK_TRY(cudaGetLastError());
-        const dim3 grid((unsigned)((nw + 127) / 128), (unsigned)nslice);
+        const dim3 grid((unsigned)((I + 8 * 128 - 1) / (8 * 128)), (unsigned)nslice);
         k_skfr_dist<<<grid, 128, 0, st>>>(bed, pitch, I, J, d_sq, d_partial);
         SK_TRY(cudaGetLastError());
         k_skfr_dist_sum<<<(unsigned)((I + 255) / 256), 256, 0, st>>>(d_partial, I, nslice, d_D);
@@ -758,7 +824,7 @@ cudaError_t skfr_run(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, in
         k_skfr_means<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(d_S, d_M, d_cnt, I, d_ab, d_nk, K, J, local,
                                                                 d_theta, d_score);
         SK_TRY(cudaGetLastError());
-        k_skfr_select<<<(unsigned)nlists, SKFR_SEL_THREADS, 0, st>>>(d_score, J, s, d_kept);
+        k_skfr_select<<<(unsigned)(nlists * SKFR_SEL_CTAS), SKFR_SEL_THREADS, 0, st>>>(d_score, J, s, d_kept);
         SK_TRY(cudaGetLastError());
         k_skfr_pairs<<<(unsigned)((K * npair + 255) / 256), 256, 0, st>>>(d_theta, d_xt, d_kept, s, local ? s : 0, K,
                                                                          J, d_pt);
