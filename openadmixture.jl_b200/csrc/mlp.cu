@@ -31,64 +31,109 @@
 
 namespace {
 
-__device__ __forceinline__ int code_of(const uint8_t *bed, int64_t pitch, int64_t i, int64_t j)
-{
-    return (bed[(size_t)j * pitch + (i >> 2)] >> ((i & 3) << 1)) & 3;
-}
-
 /* 2-bit code -> dosage: 00 -> 0, 10 -> 1, 11 -> 2, 01 (missing) -> 3 */
 __device__ __forceinline__ int8_t dosage_of(int c) { return c == 1 ? (int8_t)3 : (int8_t)(c == 0 ? 0 : c - 1); }
 
-/* allele frequency of each sketch SNP: one block per SNP */
-__global__ void k_sketch_freq(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I,
-                              const int32_t *__restrict__ snps, float *__restrict__ freq)
+/* Allele frequency of each sketch SNP: one block per SNP.  The dosage sum and the non-missing count are integers by
+ * popcount of the code bits (codes 10 and 11 have the high bit, 11 also the low one; 01 is missing), a word at a time
+ * where the columns are word-aligned. */
+__global__ void __launch_bounds__(128)
+k_sketch_freq(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, const int32_t *__restrict__ snps,
+              float *__restrict__ freq)
 {
-    __shared__ double red[8];
-    const int64_t j = snps[blockIdx.x];
-    double a = 0.0, n = 0.0;
-    for (int64_t i = threadIdx.x; i < I; i += blockDim.x) {
-        const int c = code_of(bed, pitch, i, j);
-        if (c != 1) { a += (c == 0) ? 0.0 : (double)(c - 1); n += 2.0; }
+    __shared__ double red[4];
+    const uint8_t *col = bed + (size_t)snps[blockIdx.x] * pitch;
+    const int64_t Ib = (I + 3) / 4, full = I / 4;    /* bytes; bytes without padding bits */
+    long long a = 0, n = 0;
+    auto add = [&](uint32_t v, uint32_t mask) {
+        const uint32_t lo = v & 0x55555555u & mask, hi = (v >> 1) & 0x55555555u & mask;
+        a += __popc(hi) + __popc(hi & lo);
+        n += __popc(mask & 0x55555555u) - __popc(lo & ~hi);
+    };
+    int64_t b0 = 0;
+    if ((((uintptr_t)bed | (uintptr_t)pitch) & 3u) == 0) {
+        const int64_t nw = full / 4;
+        for (int64_t w = threadIdx.x; w < nw; w += blockDim.x) add(__ldg((const uint32_t *)col + w), 0xFFFFFFFFu);
+        b0 = 4 * nw;
     }
-    const double sa = block_sum(a, red);
-    const double sn = block_sum(n, red);
+    for (int64_t b = b0 + threadIdx.x; b < Ib; b += blockDim.x)
+        add(col[b], b < full ? 0xFFu : (1u << (2 * (int)(I & 3))) - 1u);
+    const double sa = block_sum((double)a, red);
+    const double sn = block_sum(2.0 * (double)n, red);
     if (threadIdx.x == 0) freq[blockIdx.x] = sn > 0.0 ? (float)(sa / sn) : 0.5f;
 }
 
-/* dosage sketch (I x S int8) and the R standardised projections (I x R) */
-__global__ void k_sketch(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, const int32_t *__restrict__ snps,
-                         int S, const float *__restrict__ freq, int R, uint64_t seed, int8_t *__restrict__ dos,
-                         float *__restrict__ proj)
+/* Dosage sketch (I x S int8) and the R standardised projections (I x R).  A block owns the 4 individuals of one byte of
+ * the columns, a thread every 256th sketch SNP: its byte, its hash (the signs) and its standardisation serve
+ * four individuals, and the next SNP's byte is in flight while this one's 32 sums are formed.  With one individual
+ * a block, the gathers and the hash were repeated for each: 20,000 x 4,096 in 0.90 ms, now 0.45.  Bound: one FMA
+ * per cell and direction and the signs' unpacking, at the 8 warps per SM that 128 sums a thread allow. */
+constexpr int SK_THREADS = 256;
+
+__global__ void __launch_bounds__(SK_THREADS, 1)
+k_sketch(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, const int32_t *__restrict__ snps,
+         int S, const float *__restrict__ freq, int R, uint64_t seed, int8_t *__restrict__ dos,
+         float *__restrict__ proj)
 {
-    extern __shared__ float sh[];                     /* [R] partial projections per warp */
-    const int64_t i = blockIdx.x;
-    float acc[32];
+    __shared__ float sh[4][SK_THREADS / 32][32];      /* the warps' sums */
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint8_t *row = bed + blockIdx.x;
+    const int64_t i0 = (int64_t)blockIdx.x * 4;
+    const int ni = (int)min((int64_t)4, I - i0);
+    float acc[4][32];
 #pragma unroll
-    for (int r = 0; r < 32; ++r) acc[r] = 0.f;
-    for (int s = threadIdx.x; s < S; s += blockDim.x) {
-        const int c = code_of(bed, pitch, i, snps[s]);
-        const int8_t d = dosage_of(c);
-        dos[(size_t)i * S + s] = d;
-        if (d != 3) {
-            const float f = freq[s];
-            const float z = ((float)d - 2.f * f) * rsqrtf(fmaxf(2.f * f * (1.f - f), 1e-6f));
-            const uint64_t h = syn_hash3(seed, (uint64_t)s, 0);
+    for (int v = 0; v < 4; ++v)
 #pragma unroll
-            for (int r = 0; r < 32; ++r)
-                if (r < R) acc[r] += ((h >> r) & 1u) ? z : -z;
+        for (int r = 0; r < 32; ++r) acc[v][r] = 0.f;
+    uint32_t byte = 0u;
+    int32_t next = 0;
+    float f = 0.f, fn = 0.f;
+    if (tid < S) {
+        byte = row[(size_t)snps[tid] * pitch];
+        f = freq[tid];
+    }
+    if (tid + SK_THREADS < S) next = snps[tid + SK_THREADS];
+    for (int s = tid; s < S; s += SK_THREADS) {
+        uint32_t bn = 0u;
+        if (s + SK_THREADS < S) {
+            bn = row[(size_t)next * pitch];
+            fn = freq[s + SK_THREADS];
         }
+        if (s + 2 * SK_THREADS < S) next = snps[s + 2 * SK_THREADS];
+        const float w = rsqrtf(fmaxf(2.f * f * (1.f - f), 1e-6f));
+        const uint32_t h = (uint32_t)syn_hash3(seed, (uint64_t)s, 0);
+        float z[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const uint32_t c = (byte >> (2 * v)) & 3u;
+            const int8_t d = dosage_of((int)c);
+            if (v < ni) dos[(size_t)(i0 + v) * S + s] = d;
+            z[v] = c == 1u ? 0.f : ((float)d - 2.f * f) * w;   /* a missing dosage adds 0 to every sum */
+        }
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+            const float sg = __uint_as_float(0xBF800000u ^ ((h << (31 - r)) & 0x80000000u));   /* bit r: +1, else -1 */
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[v][r] = fmaf(z[v], sg, acc[v][r]);
+        }
+        byte = bn;
+        f = fn;
     }
-    const float scale = rsqrtf((float)S);
-    for (int r = 0; r < R; ++r) {
-        float v = acc[r];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) sh[(threadIdx.x >> 5) * R + r] = v;
-    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+            float x = acc[v][r];
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            if (lane == 0) sh[v][warp][r] = x;
+        }
     __syncthreads();
-    if (threadIdx.x < R) {
-        float v = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sh[w * R + threadIdx.x];
-        proj[(size_t)i * R + threadIdx.x] = v * scale;
+    const float scale = rsqrtf((float)S);
+    const int v = tid >> 5;
+    if (v < ni && lane < R) {
+        float x = 0.f;
+        for (int w = 0; w < SK_THREADS / 32; ++w) x += sh[v][w][lane];
+        proj[(size_t)(i0 + v) * R + lane] = x * scale;
     }
 }
 
@@ -100,36 +145,97 @@ extern "C" int admix_sketch(const uint8_t *d_bed, int64_t pitch, int64_t I, cons
     if (!d_bed || !d_snps || !d_freq || !d_dos || !d_proj || I < 1 || S < 1 || R < 0 || R > 32 || pitch < (I + 3) / 4)
         return ADMIX_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    k_sketch_freq<<<S, 256, 0, st>>>(d_bed, pitch, I, d_snps, d_freq);
-    k_sketch<<<(unsigned)I, 256, sizeof(float) * 8 * (R > 0 ? R : 1), st>>>(d_bed, pitch, I, d_snps, S, d_freq, R,
-                                                                            seed, d_dos, d_proj);
+    k_sketch_freq<<<S, 128, 0, st>>>(d_bed, pitch, I, d_snps, d_freq);
+    k_sketch<<<(unsigned)((I + 3) / 4), SK_THREADS, 0, st>>>(d_bed, pitch, I, d_snps, S, d_freq, R, seed, d_dos, d_proj);
     return cudaGetLastError() == cudaSuccess ? ADMIX_OK : ADMIX_ERR_CUDA;
 }
 
 namespace {
 
-/* ---- operand loaders: element (r, c) of a logical row-major matrix ---- */
-struct LoadF {                     /* dense FP32 with arbitrary strides (transposes are strides) */
+/* ---- operand loaders: row r of an operand, 8 consecutive elements of the reduction from c0 (a multiple of 8).  load()
+ * only reads memory, so that a slice's reads are all in flight together and a slice ahead of their use;
+ * values() turns them into numbers, zero past the operand's bounds. ---- */
+struct LoadF {                     /* dense FP32: element (r, c) at p[r * sr + c * sc] */
     const float *p; int64_t sr, sc;
-    __device__ float operator()(int64_t r, int64_t c) const { return p[r * sr + c * sc]; }
-};
-struct LoadX {                     /* network input: [dosage - 2f (0 if missing) | projections] */
-    const int8_t *dos; const float *center; const float *proj; int S, R;
-    __device__ float operator()(int64_t m, int64_t k) const
+    struct Raw { float v[8]; };
+    __device__ __forceinline__ void load(Raw &w, int64_t r, int64_t c0, int64_t rows, int64_t cols) const
     {
-        if (k < S) {
-            const int8_t d = dos[m * S + k];
-            return d == 3 ? 0.f : (float)d - center[k];
+        const float *q = p + r * sr + c0 * sc;
+        if (sc == 1 && (((uintptr_t)p | (uintptr_t)(sr * 4)) & 15u) == 0 && r < rows && c0 + 8 <= cols) {
+            const float4 a = *(const float4 *)q, b = *(const float4 *)(q + 4);
+            w.v[0] = a.x; w.v[1] = a.y; w.v[2] = a.z; w.v[3] = a.w;
+            w.v[4] = b.x; w.v[5] = b.y; w.v[6] = b.z; w.v[7] = b.w;
+            return;
         }
-        return proj[m * R + (k - S)];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w.v[e] = (r < rows && c0 + e < cols) ? q[e * sc] : 0.f;
+    }
+    __device__ __forceinline__ void values(float (&v)[8], const Raw &w, int64_t, int64_t, int64_t, int64_t) const
+    {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = w.v[e];
     }
 };
-struct LoadXT {                    /* the input transposed: (k, m) */
+/* the network input [dosage - 2f (0 if missing) | projections]; a dosage byte or a projection's bits per element */
+struct LoadX {                     /* row = individual, reduction = feature */
+    const int8_t *dos; const float *center; const float *proj; int S, R;
+    struct Raw { uint32_t v[8]; };
+    __device__ __forceinline__ void load(Raw &w, int64_t m, int64_t k0, int64_t rows, int64_t cols) const
+    {
+        if (m < rows && k0 + 8 <= S && (((uintptr_t)dos | (uintptr_t)S) & 7u) == 0) {
+            const uint2 x = *(const uint2 *)(dos + m * S + k0);   /* k0 is a multiple of 8 */
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w.v[e] = ((e < 4 ? x.x : x.y) >> (8 * (e & 3))) & 0xFFu;
+            return;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int64_t k = k0 + e;
+            w.v[e] = 0u;
+            if (m < rows && k < cols) w.v[e] = k < S ? (uint32_t)(uint8_t)dos[m * S + k] : __float_as_uint(proj[m * R + (k - S)]);
+        }
+    }
+    __device__ __forceinline__ void values(float (&v)[8], const Raw &w, int64_t m, int64_t k0, int64_t rows, int64_t cols) const
+    {
+        if (k0 + 8 <= S) {
+            float c[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) c[e] = __ldg(center + k0 + e);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = (m < rows && w.v[e] != 3u) ? (float)(int8_t)w.v[e] - c[e] : 0.f;
+            return;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int64_t k = k0 + e;
+            if (k < S) v[e] = (m < rows && w.v[e] != 3u) ? (float)(int8_t)w.v[e] - __ldg(center + k) : 0.f;
+            else v[e] = __uint_as_float(w.v[e]);
+        }
+    }
+};
+struct LoadXT {                    /* row = feature, reduction = individual */
     LoadX x;
-    __device__ float operator()(int64_t k, int64_t m) const { return x(m, k); }
+    struct Raw { uint32_t v[8]; };
+    __device__ __forceinline__ void load(Raw &w, int64_t k, int64_t m0, int64_t rows, int64_t cols) const
+    {
+        if (k < x.S) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w.v[e] = m0 + e < cols ? (uint32_t)(uint8_t)x.dos[(m0 + e) * x.S + k] : 3u;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w.v[e] = (k < rows && m0 + e < cols) ? __float_as_uint(x.proj[(m0 + e) * x.R + (k - x.S)]) : 0u;
+        }
+    }
+    __device__ __forceinline__ void values(float (&v)[8], const Raw &w, int64_t k, int64_t, int64_t, int64_t) const
+    {
+        const float c = k < x.S ? __ldg(x.center + k) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = k < x.S ? (w.v[e] == 3u ? 0.f : (float)(int8_t)w.v[e] - c) : __uint_as_float(w.v[e]);
+    }
 };
 
 constexpr int GT_M = 128, GT_N = 64, GT_K = 32;   /* output tile rows x columns, reduction slice */
+constexpr int GT_THREADS = 512;
 constexpr int GT_D = 4;                             /* slices per fresh accumulation */
 constexpr uint32_t GT_WAIT = 1u << 22;              /* polls of a bounded wait */
 /* one stage: A hi, A lo (128 x 32 BF16, K-major core matrices), B hi, B lo (64 x 32) */
@@ -138,19 +244,31 @@ constexpr uint32_t GT_STAGE = 2 * GT_A + 2 * GT_B;
 constexpr uint32_t GT_SMEM = 2 * GT_STAGE + 1024;
 constexpr uint32_t GT_A_LBO = GT_M * 16, GT_B_LBO = GT_N * 16;
 
-/* v = hi + lo, both BF16 (hi rounded to nearest, lo the BF16 of the remainder) */
-__device__ __forceinline__ void split_bf16(float v, uint32_t &hi, uint32_t &lo)
+/* 8 values as BF16 high parts (rounded to nearest) and the BF16 of the remainders, v = hi + lo, packed in pairs */
+__device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo)
 {
-    hi = pack_bf16x2(v, 0.f) & 0xFFFFu;
-    lo = pack_bf16x2(v - __uint_as_float(hi << 16), 0.f) & 0xFFFFu;
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        h[e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+        l[e] = pack_bf16x2(v[2 * e] - __uint_as_float(h[e] << 16), v[2 * e + 1] - __uint_as_float(h[e] & 0xFFFF0000u));
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
 /* C[m, n] = alpha * sum_k A(m, k) B(k, n) (+ bias[n]); relu if act; times [mask(m, n) > 0] if mask.
- * 128 threads, one 128 x 64 output tile per CTA (thread = output row = TMEM lane).  Two smem
- * stages: the threads load slice c+1 while the tensor core multiplies slice c.  Every wait is
+ * 512 threads, one 128 x 64 output tile per CTA: thread t owns output row (TMEM lane) 32 (warp % 4) + lane and the 16
+ * columns from 16 (warp / 4), and converts one granule of A (row t % 128) and, for t < 256, one of B.  Two smem
+ * stages: the threads convert slice c+1 while the tensor core multiplies slice c, and the global reads of
+ * slice c+2 are in flight meanwhile.  B is given by its rows: element (n, k) of loader B is B(k, n).
+ * Bound: the operands' conversion on the CUDA cores, at the latency of one slice where the grid is small (hence 12
+ * elements a thread).  128 threads that read each of their 48 elements where they converted it put 48 memory
+ * latencies in series: the encoder's first layer on 20,000
+ * individuals took 2.78 ms, its weight gradient on 4,096 2.27 ms; now 0.75 and 0.20.  Every wait is
  * bounded; a CTA whose wait runs out writes NaN into its tile (the failure shows in the loss). */
 template <class LA, class LB>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(GT_THREADS, 2)
 k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *__restrict__ bias, int act,
           const float *__restrict__ mask, float *__restrict__ C, int64_t ldc)
 {
@@ -172,7 +290,8 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = tmem_holder;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    const int col0 = 16 * (warp >> 2);
+    const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     bool ok = true;
     auto wait = [&](uint64_t *b, uint32_t parity) {
         if (!ok) return;
@@ -183,68 +302,47 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
         ok = false;
         abort_flag = 1;
     };
-    float acc[GT_N];
+    float acc[16];
 #pragma unroll
-    for (int n = 0; n < GT_N; ++n) acc[n] = 0.f;
+    for (int n = 0; n < 16; ++n) acc[n] = 0.f;
     auto drain = [&]() {   /* the finished accumulation block into the FP32 registers */
         tc_fence_after_sync();
+        float v[16];
+        tmem_ld16(my_tmem, v);
 #pragma unroll
-        for (int c0 = 0; c0 < GT_N; c0 += 16) {
-            float v[16];
-            tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) acc[c0 + e] += v[e];
-        }
+        for (int e = 0; e < 16; ++e) acc[e] += v[e];
     };
     const int nch = (int)((Kd + GT_K - 1) / GT_K);
     constexpr uint32_t idesc = idesc_bf16_f32(GT_M, GT_N);
+    typename LA::Raw ra;
+    typename LB::Raw rb;
+    const int am = tid & (GT_M - 1), ag = tid >> 7, bn = tid & (GT_N - 1), bg = tid >> 6;
+    const bool hasb = tid < GT_N * GT_K / 8;
+    static_assert(GT_M * GT_K / 8 == GT_THREADS, "one granule of A a thread");
+    auto fetch = [&](int c) {
+        const int64_t k0 = (int64_t)c * GT_K;
+        A.load(ra, m0 + am, k0 + 8 * ag, M, Kd);
+        if (hasb) B.load(rb, n0 + bn, k0 + 8 * bg, N, Kd);
+    };
+    if (nch > 0) fetch(0);
     for (int c = 0; c < nch; ++c) {
         const int st = c & 1;
         uint8_t *Ah = sm + st * GT_STAGE, *Al = Ah + GT_A, *Bh = Al + GT_A, *Bl = Bh + GT_B;
         if (c >= 2) wait(&bar[st], (uint32_t)(((c - 2) >> 1) & 1));   /* stage st is free again */
         const int64_t k0 = (int64_t)c * GT_K;
-        /* A: thread t loads row m0 + t of the slice, 4 granules of 8 */
-        {
-            const int64_t m = m0 + tid;
-#pragma unroll
-            for (int gr = 0; gr < GT_K / 8; ++gr) {
-                uint32_t h[4], l[4];
-#pragma unroll
-                for (int e = 0; e < 8; e += 2) {
-                    const int64_t ka = k0 + 8 * gr + e;
-                    const float v0 = (m < M && ka < Kd) ? A(m, ka) : 0.f;
-                    const float v1 = (m < M && ka + 1 < Kd) ? A(m, ka + 1) : 0.f;
-                    uint32_t h0, l0, h1, l1;
-                    split_bf16(v0, h0, l0);
-                    split_bf16(v1, h1, l1);
-                    h[e / 2] = h0 | (h1 << 16);
-                    l[e / 2] = l0 | (l1 << 16);
-                }
-                *(uint4 *)(Ah + gr * GT_A_LBO + 16 * tid) = make_uint4(h[0], h[1], h[2], h[3]);
-                *(uint4 *)(Al + gr * GT_A_LBO + 16 * tid) = make_uint4(l[0], l[1], l[2], l[3]);
-            }
+        float v[8];
+        uint4 h, l;
+        A.values(v, ra, m0 + am, k0 + 8 * ag, M, Kd);
+        split8(v, h, l);
+        *(uint4 *)(Ah + ag * GT_A_LBO + 16 * am) = h;
+        *(uint4 *)(Al + ag * GT_A_LBO + 16 * am) = l;
+        if (hasb) {
+            B.values(v, rb, n0 + bn, k0 + 8 * bg, N, Kd);
+            split8(v, h, l);
+            *(uint4 *)(Bh + bg * GT_B_LBO + 16 * bn) = h;
+            *(uint4 *)(Bl + bg * GT_B_LBO + 16 * bn) = l;
         }
-        /* B: 64 columns x 4 granules = 256 tasks, two per thread; B row n holds B(k, n0 + n) */
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int task = tid + 128 * u;
-            const int n = task & (GT_N - 1), gr = task >> 6;
-            const int64_t col = n0 + n;
-            uint32_t h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-                const int64_t ka = k0 + 8 * gr + e;
-                const float v0 = (col < N && ka < Kd) ? B(ka, col) : 0.f;
-                const float v1 = (col < N && ka + 1 < Kd) ? B(ka + 1, col) : 0.f;
-                uint32_t h0, l0, h1, l1;
-                split_bf16(v0, h0, l0);
-                split_bf16(v1, h1, l1);
-                h[e / 2] = h0 | (h1 << 16);
-                l[e / 2] = l0 | (l1 << 16);
-            }
-            *(uint4 *)(Bh + gr * GT_B_LBO + 16 * n) = make_uint4(h[0], h[1], h[2], h[3]);
-            *(uint4 *)(Bl + gr * GT_B_LBO + 16 * n) = make_uint4(l[0], l[1], l[2], l[3]);
-        }
+        if (c + 1 < nch) fetch(c + 1);
         fence_async_smem();
         if (c > 0 && c % GT_D == 0) {   /* the block ending at slice c-1: its MMAs done, into registers */
             wait(&bar[(c - 1) & 1], (uint32_t)(((c - 1) >> 1) & 1));
@@ -278,11 +376,11 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
         mbar_wait_bounded(&bar[0], 0u, 1024u); mbar_wait_bounded(&bar[0], 1u, 1024u);
         mbar_wait_bounded(&bar[1], 0u, 1024u); mbar_wait_bounded(&bar[1], 1u, 1024u);
     }
-    const int64_t m = m0 + tid;
+    const int64_t m = m0 + 32 * (warp & 3) + (tid & 31);
     if (m < M) {
 #pragma unroll
-        for (int n = 0; n < GT_N; ++n) {
-            const int64_t col = n0 + n;
+        for (int n = 0; n < 16; ++n) {
+            const int64_t col = n0 + col0 + n;
             if (col >= N) break;
             float v = alpha * acc[n] + (bias ? bias[col] : 0.f);
             if (act) v = fmaxf(v, 0.f);
@@ -306,7 +404,7 @@ cudaError_t gemm(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, cons
         ready = true;
     }
     dim3 grid((unsigned)((N + GT_N - 1) / GT_N), (unsigned)((M + GT_M - 1) / GT_M));
-    k_gemm_tc<LA, LB><<<grid, 128, GT_SMEM, st>>>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc);
+    k_gemm_tc<LA, LB><<<grid, GT_THREADS, GT_SMEM, st>>>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc);
     return cudaGetLastError();
 }
 
@@ -371,65 +469,139 @@ cudaError_t colsum(const float *dY, int64_t M, int64_t N, float *db, cudaStream_
 }
 
 /* closed-form P step from Q: p_kj = sum_i nm q_ki g_ij / (2 sum_i nm q_ki), clamped to
- * [1e-5, 1-1e-5] like project_p! (projections.jl:69-74).  Thread = SNP; q staged through shared
- * memory 64 individuals at a time as (k, k+1) pairs, both sums accumulated in FP32 pairs (one
- * paired FMA per k pair and cell); a missing cell adds zeros, so no thread branches on the
- * genotype, and one byte load serves four cells.  Each sum is the same per-k FP32 sequence as
- * a per-cell loop that skips the missing cells. */
-template <int K>
-__global__ void __launch_bounds__(128)
+ * [1e-5, 1-1e-5] like project_p! (projections.jl:69-74).  A thread owns two SNPs, one in each half of its paired
+ * FP32 sums; q is staged through shared memory 64 individuals at a time with each value twice, so a pair of cells
+ * takes one paired FMA per cluster and sum and no duplication of the genotype factors, which a table gives per code
+ * pair.  A missing cell adds zeros, so no thread branches on the genotype.  Each sum is the same per-k FP32 sequence
+ * as a per-cell loop that skips the missing cells.  W = 8: columns aligned to 8 bytes; otherwise
+ * aligned words, shifted.
+ * Bound: instruction issue at the few warps that J / 2 threads are (the sums of a SNP are serial chains over the
+ * individuals).  I=20k, J=100k, K=8: 2.53 ms with one SNP a thread and a byte per load, 1.88 now; two pairs a
+ * thread, or the clusters split over two threads, repeat the staging or the decoding and take 2.35 to 2.46. */
+template <int K, int W>
+__global__ void __launch_bounds__(64)
 k_warm_p(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, int64_t J, const double *__restrict__ q,
          double *__restrict__ p)
 {
-    constexpr int KH = (K + 1) / 2;                  /* k pairs (odd K: the last pair's second half is 0) */
-    __shared__ __align__(16) float2 qs[64 * KH];
-    const int64_t j = (int64_t)blockIdx.x * 128 + threadIdx.x;
-    const uint8_t *col = bed + (size_t)(j < J ? j : 0) * pitch;
-    float2 num[KH], den[KH];   /* sum_i q_ki g_ij and sum_i nm q_ki */
+    constexpr int K2 = (K + 1) / 2;                  /* 16-byte groups of two doubled values per individual */
+    __shared__ __align__(16) float4 qs[64 * K2];
+    const int64_t ja = ((int64_t)blockIdx.x * 64 + threadIdx.x) * 2, jb = ja + 1;
+    const uint8_t *ca = bed + (size_t)(ja < J ? ja : 0) * pitch, *cb = bed + (size_t)(jb < J ? jb : 0) * pitch;
+    const int64_t Ib = (I + 3) / 4;
+    float2 num[2 * K2], den[2 * K2];                  /* (SNP a, SNP b): sum_i q_ki g_ij and sum_i nm q_ki */
 #pragma unroll
-    for (int kh = 0; kh < KH; ++kh) num[kh] = den[kh] = make_float2(0.f, 0.f);
-    for (int64_t i0 = 0; i0 < I; i0 += 64) {
-        const int n = (int)min((int64_t)64, I - i0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < 64 * KH; t += 128) {
-            const int ii = t / KH, k = 2 * (t - ii * KH);
-            float a = 0.f, b = 0.f;
-            if (ii < n) {
-                a = (float)q[(size_t)K * (i0 + ii) + k];
-                if (k + 1 < K) b = (float)q[(size_t)K * (i0 + ii) + k + 1];
+    for (int k = 0; k < 2 * K2; ++k) num[k] = den[k] = make_float2(0.f, 0.f);
+    /* factors by code pair (code of a | code of b << 2): (g_a, g_b) and (nm_a, nm_b) as BF16 pairs (exact), 16 copies
+     * so that a half-warp's 8-byte loads never share a bank */
+    __shared__ __align__(16) uint2 tab[16 * 16];
+    for (int t = threadIdx.x; t < 256; t += 64) {
+        const uint32_t c0 = (uint32_t)(t >> 4) & 3u, c1 = (uint32_t)(t >> 6);
+        auto gf = [](uint32_t c) { return c == 3u ? 2.f : (c == 2u ? 1.f : 0.f); };   /* codes 00 -> 0, 10 -> 1, 11 -> 2 */
+        auto mf = [](uint32_t c) { return c == 1u ? 0.f : 1.f; };                      /* 01: missing */
+        tab[t] = make_uint2(pack_bf16x2(gf(c0), gf(c1)), pack_bf16x2(mf(c0), mf(c1)));
+    }
+    const uint8_t *tl = (const uint8_t *)tab + 8 * (threadIdx.x & 15);
+    /* 8 two-bit codes spread to the low halves of 8 nibbles */
+    auto spread = [](uint32_t x) {
+        x = (x | (x << 8)) & 0x00FF00FFu;
+        x = (x | (x << 4)) & 0x0F0F0F0Fu;
+        return (x | (x << 2)) & 0x33333333u;
+    };
+    /* the 16 bytes of 64 individuals of a column, missing past its end */
+    auto codes = [&](const uint8_t *col, int64_t i0, uint32_t (&w)[4]) {
+        const int64_t b0 = i0 >> 2;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) w[v] = 0x55555555u;
+        if (b0 + 16 <= Ib) {
+            if (W == 8) {
+                const uint2 x = __ldg((const uint2 *)(col + b0)), y = __ldg((const uint2 *)(col + b0) + 1);
+                w[0] = x.x; w[1] = x.y; w[2] = y.x; w[3] = y.y;
+            } else {   /* the aligned words that hold the 16 bytes, each with at least one of them */
+                const uint32_t mis = (uint32_t)((uintptr_t)(col + b0) & 3u);
+                const uint32_t *al = (const uint32_t *)(col + b0 - mis);
+                uint32_t x[5];
+#pragma unroll
+                for (int v = 0; v < 5; ++v) x[v] = (v < 4 || mis) ? __ldg(al + v) : 0u;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) w[v] = __funnelshift_r(x[v], x[v + 1], 8 * mis);
             }
-            qs[t] = make_float2(a, b);
+        } else {
+#pragma unroll
+            for (int n = 0; n < 16; ++n)
+                if (b0 + n < Ib) w[n >> 2] = (w[n >> 2] & ~(0xFFu << (8 * (n & 3)))) | ((uint32_t)__ldg(col + b0 + n) << (8 * (n & 3)));
         }
+    };
+    /* this thread's q values of the next 64 individuals; 0 past I, which adds nothing whatever the codes there */
+    float qa[K2], qb[K2];
+    auto fetch = [&](int64_t i0) {
+#pragma unroll
+        for (int e = 0; e < K2; ++e) {
+            const int t = threadIdx.x + e * 64, ii = t / K2, k = 2 * (t - ii * K2);
+            const double *src = q + (size_t)K * (i0 + ii) + k;
+            qa[e] = i0 + ii < I ? (float)src[0] : 0.f;
+            qb[e] = (i0 + ii < I && k + 1 < K) ? (float)src[1] : 0.f;
+        }
+    };
+    uint32_t wa[4], wb[4];
+    codes(ca, 0, wa);
+    codes(cb, 0, wb);
+    fetch(0);
+    for (int64_t i0 = 0; i0 < I; i0 += 64) {
         __syncthreads();
-        if (j < J) {
-            for (int ib = 0; 4 * ib < n; ++ib) {
-                const uint32_t byte = col[(size_t)(i0 >> 2) + ib];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int ii = 4 * ib + t;
-                    if (ii >= n) break;
-                    const uint32_t c = (byte >> (2 * t)) & 3u;
-                    const float g = c == 3u ? 2.f : (c == 2u ? 1.f : 0.f);   /* codes 00 -> 0, 10 -> 1, 11 -> 2 */
-                    const float nm = c == 1u ? 0.f : 1.f;                    /* 01: missing */
-                    const float2 g2 = make_float2(g, g), n2 = make_float2(nm, nm);
+        for (int e = 0; e < K2; ++e) qs[threadIdx.x + e * 64] = make_float4(qa[e], qa[e], qb[e], qb[e]);
+        __syncthreads();
+        uint32_t na[4] = {wa[0], wa[1], wa[2], wa[3]}, nb[4] = {wb[0], wb[1], wb[2], wb[3]};
+        if (i0 + 64 < I) {
+            fetch(i0 + 64);
+            codes(ca, i0 + 64, na);
+            codes(cb, i0 + 64, nb);
+        }
 #pragma unroll
-                    for (int kh = 0; kh < KH; ++kh) {
-                        const float2 qv = qs[ii * KH + kh];
-                        num[kh] = __ffma2_rn(qv, g2, num[kh]);
-                        den[kh] = __ffma2_rn(qv, n2, den[kh]);
+        for (int v = 0; v < 4; ++v) {
+#pragma unroll 1
+            for (int hw = 0; hw < 2; ++hw) {
+                const uint32_t x = spread((wa[v] >> (16 * hw)) & 0xFFFFu) | (spread((wb[v] >> (16 * hw)) & 0xFFFFu) << 2);
+                const float4 *qv = qs + (16 * v + 8 * hw) * K2;
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    const uint2 f = *(const uint2 *)(tl + ((t < 2 ? x << (7 - 4 * t) : x >> (4 * t - 7)) & 0x780u));
+                    const float2 g = make_float2(__uint_as_float(f.x << 16), __uint_as_float(f.x & 0xFFFF0000u));
+                    const float2 m = make_float2(__uint_as_float(f.y << 16), __uint_as_float(f.y & 0xFFFF0000u));
+#pragma unroll
+                    for (int h = 0; h < K2; ++h) {
+                        const float4 y = qv[t * K2 + h];
+                        const float2 y0 = make_float2(y.x, y.y), y1 = make_float2(y.z, y.w);
+                        num[2 * h] = __ffma2_rn(y0, g, num[2 * h]);
+                        den[2 * h] = __ffma2_rn(y0, m, den[2 * h]);
+                        if (2 * h + 1 < K) {
+                            num[2 * h + 1] = __ffma2_rn(y1, g, num[2 * h + 1]);
+                            den[2 * h + 1] = __ffma2_rn(y1, m, den[2 * h + 1]);
+                        }
                     }
                 }
             }
         }
-    }
-    if (j < J)
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const float nk = (k & 1) ? num[k >> 1].y : num[k >> 1].x;
-            const float dk = 2.f * ((k & 1) ? den[k >> 1].y : den[k >> 1].x);
-            const double v = dk > 0.f ? (double)nk / (double)dk : 0.5;
-            p[(size_t)K * j + k] = fmin(fmax(v, 1e-5), 1.0 - 1e-5);
-        }
+        for (int v = 0; v < 4; ++v) { wa[v] = na[v]; wb[v] = nb[v]; }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const float na = num[k].x, da = 2.f * den[k].x, nb = num[k].y, db = 2.f * den[k].y;
+        const double va = da > 0.f ? (double)na / (double)da : 0.5, vb = db > 0.f ? (double)nb / (double)db : 0.5;
+        if (ja < J) p[(size_t)K * ja + k] = fmin(fmax(va, 1e-5), 1.0 - 1e-5);
+        if (jb < J) p[(size_t)K * jb + k] = fmin(fmax(vb, 1e-5), 1.0 - 1e-5);
+    }
+}
+
+template <int K>
+cudaError_t launch_warm_p(const uint8_t *bed, int64_t pitch, int64_t I, int64_t J, const double *q, double *p, cudaStream_t st)
+{
+    const unsigned grid = (unsigned)((J + 127) / 128);
+    const uintptr_t al = (uintptr_t)bed | (uintptr_t)pitch;
+    if ((al & 7u) == 0) k_warm_p<K, 8><<<grid, 64, 0, st>>>(bed, pitch, I, J, q, p);
+    else k_warm_p<K, 1><<<grid, 64, 0, st>>>(bed, pitch, I, J, q, p);
+    return cudaGetLastError();
 }
 
 } // namespace
@@ -442,10 +614,10 @@ int admix_mlp_forward(const admix_mlp *net, int64_t n, const int8_t *dos, const 
     if (!net || n < 1 || !dos || !center || !proj || !h1 || !h2 || !logits || !probs) return ADMIX_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t D = net->S + net->R, H = net->H, K = net->K;
-    cudaError_t e = gemm(LoadX{dos, center, proj, net->S, net->R}, LoadF{net->w1, H, 1}, n, H, D, 1.f, net->b1, 1,
+    cudaError_t e = gemm(LoadX{dos, center, proj, net->S, net->R}, LoadF{net->w1, 1, H}, n, H, D, 1.f, net->b1, 1,
                          nullptr, h1, H, st);
-    if (e == cudaSuccess) e = gemm(LoadF{h1, H, 1}, LoadF{net->w2, H, 1}, n, H, H, 1.f, net->b2, 1, nullptr, h2, H, st);
-    if (e == cudaSuccess) e = gemm(LoadF{h2, H, 1}, LoadF{net->w3, K, 1}, n, K, H, 1.f, net->b3, 0, nullptr, logits, K, st);
+    if (e == cudaSuccess) e = gemm(LoadF{h1, H, 1}, LoadF{net->w2, 1, H}, n, H, H, 1.f, net->b2, 1, nullptr, h2, H, st);
+    if (e == cudaSuccess) e = gemm(LoadF{h2, H, 1}, LoadF{net->w3, 1, K}, n, K, H, 1.f, net->b3, 0, nullptr, logits, K, st);
     if (e == cudaSuccess) {
         k_softmax_ce<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(logits, n, (int)K, probs, nullptr, nullptr, nullptr);
         e = cudaGetLastError();
@@ -464,16 +636,16 @@ int admix_mlp_backward(const admix_mlp *net, const admix_mlp_grads *grad, int64_
     k_softmax_ce<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(logits, n, (int)K, probs, target, dlogits, loss);
     cudaError_t e = cudaGetLastError();
     /* layer 3 */
-    if (e == cudaSuccess) e = gemm(LoadF{h2, 1, H}, LoadF{dlogits, K, 1}, H, K, n, 1.f, nullptr, 0, nullptr, grad->w3, K, st);
+    if (e == cudaSuccess) e = gemm(LoadF{h2, 1, H}, LoadF{dlogits, 1, K}, H, K, n, 1.f, nullptr, 0, nullptr, grad->w3, K, st);
     if (e == cudaSuccess) e = colsum(dlogits, n, K, grad->b3, st);
-    if (e == cudaSuccess) e = gemm(LoadF{dlogits, K, 1}, LoadF{net->w3, 1, K}, n, H, K, 1.f, nullptr, 0, h2, dh2, H, st);
+    if (e == cudaSuccess) e = gemm(LoadF{dlogits, K, 1}, LoadF{net->w3, K, 1}, n, H, K, 1.f, nullptr, 0, h2, dh2, H, st);
     /* layer 2 */
-    if (e == cudaSuccess) e = gemm(LoadF{h1, 1, H}, LoadF{dh2, H, 1}, H, H, n, 1.f, nullptr, 0, nullptr, grad->w2, H, st);
+    if (e == cudaSuccess) e = gemm(LoadF{h1, 1, H}, LoadF{dh2, 1, H}, H, H, n, 1.f, nullptr, 0, nullptr, grad->w2, H, st);
     if (e == cudaSuccess) e = colsum(dh2, n, H, grad->b2, st);
-    if (e == cudaSuccess) e = gemm(LoadF{dh2, H, 1}, LoadF{net->w2, 1, H}, n, H, H, 1.f, nullptr, 0, h1, dh1, H, st);
+    if (e == cudaSuccess) e = gemm(LoadF{dh2, H, 1}, LoadF{net->w2, H, 1}, n, H, H, 1.f, nullptr, 0, h1, dh1, H, st);
     /* layer 1 */
     if (e == cudaSuccess)
-        e = gemm(LoadXT{LoadX{dos, center, proj, net->S, net->R}}, LoadF{dh1, H, 1}, D, H, n, 1.f, nullptr, 0, nullptr,
+        e = gemm(LoadXT{LoadX{dos, center, proj, net->S, net->R}}, LoadF{dh1, 1, H}, D, H, n, 1.f, nullptr, 0, nullptr,
                  grad->w1, H, st);
     if (e == cudaSuccess) e = colsum(dh1, n, H, grad->b1, st);
     return e == cudaSuccess ? ADMIX_OK : ADMIX_ERR_CUDA;
@@ -495,9 +667,7 @@ int admix_warm_p(const uint8_t *d_bed, int64_t pitch, int64_t I, int64_t J, int3
     if (!d_bed || !d_q || !d_p || I < 1 || J < 1 || K < 1 || K > ADMIX_MAX_K || pitch < (I + 3) / 4)
         return ADMIX_ERR_ARG;
     cudaError_t e = cudaErrorInvalidValue;
-    ADMIX_DISPATCH_K(K, (k_warm_p<KK><<<(unsigned)((J + 127) / 128), 128, 0, (cudaStream_t)stream>>>(d_bed, pitch, I, J,
-                                                                                                  d_q, d_p),
-                         e = cudaGetLastError()));
+    ADMIX_DISPATCH_K(K, e = launch_warm_p<KK>(d_bed, pitch, I, J, d_q, d_p, (cudaStream_t)stream));
     return e == cudaSuccess ? ADMIX_OK : ADMIX_ERR_CUDA;
 }
 
