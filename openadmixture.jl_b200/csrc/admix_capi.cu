@@ -57,7 +57,7 @@ struct admix_ctx {
     int32_t *iter_host = &iter_store;
     unsigned long long *counts = nullptr;
     LoglikPlan llp;
-    SweepPlan sq, sp, sqm, spm, llm; /* *m: mixed-precision Q sweep, P sweep, loglik */
+    SweepPlan sq, sp, sqm, spm, llm, epm; /* *m: mixed-precision Q sweep, P sweep, loglik */
     int64_t cap_sq = 1, cap_sp = 1, cap_sqm = 1, cap_spm = 1, cap_llm = 1;   /* slice counts the partial buffers hold */
     QNPlan qnp;
     size_t bytes = 0;
@@ -193,6 +193,8 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
     h->cap_sp = h->sp.S;
     h->cap_sqm = h->sqm.S;
     h->cap_spm = h->spm.S;
+    /* the EM sums' rows are 2 K long, the sweep's K (K + 3) / 2 */
+    h->epm = plan_em_p_mixed(K, I, J, h->sms, h->cap_spm * (K + 3) / 4);
     h->cap_llm = h->llm.S;
 
     Carver mem;
@@ -448,14 +450,15 @@ static cudaError_t enq_sweep_p_mode(admix_ctx *h, int mode, int wq, int wp, int 
     const bool mx = (mode == 0 && (h->flags & ADMIX_FLAG_MIXED)) || mode == 2;
     /* entries per SNP: T + K (gradient / Hessian) or 2K (EM sums) */
     const size_t row = (size_t)(mode == 0 ? h->K * (h->K + 1) / 2 + h->K : 2 * h->K);
-    *S = h->streamed ? 1 : (mx ? h->spm.S : h->sp.S);
+    *S = h->streamed ? 1 : (mode == 2 ? h->epm.S : mx ? h->spm.S : h->sp.S);
     return for_blocks(h, [&](const uint8_t *bed, int64_t j0, int64_t nj, int b) -> cudaError_t {
         (void)b;
         const double *P = Pof(h, wp) + (size_t)h->K * j0;
         double *out = h->parts_p + (size_t)j0 * row;
         if (mx) {
-            const SweepPlan pl = h->streamed ? block_plan(plan_sweep_p_mixed(h->K, h->I, nj, h->sms), (h->I + 31) / 32 * 32)
-                                             : h->spm;
+            const auto plan = mode == 2 ? plan_em_p_mixed : plan_sweep_p_mixed;
+            const SweepPlan pl = h->streamed ? block_plan(plan(h->K, h->I, nj, h->sms, INT64_MAX), (h->I + 31) / 32 * 32)
+                                             : mode == 2 ? h->epm : h->spm;
             return launch_sweep_p_mixed(h->K, mode == 2 ? 1 : 0, bed, h->I, nj, h->pitch, Qof(h, wq), P, pl, out,
                                         &h->sc->tc_err, h->pkg, h->st);
         }
@@ -498,8 +501,8 @@ static cudaError_t enq_em(admix_ctx *h)
 {
     /* em_q! then em_p! (mode :base, both from (q, p)), then p, q <- next (algorithms_outer.jl:23-30).
      * The EM Q-step's sums are the Q-side gradient, so the mixed form takes them from its
-     * tensor-core gradient / Hessian sweep; its P-step sums come from the EM mode of the mixed
-     * P pipeline (FP32 cells, FP64 across chunks). */
+     * tensor-core gradient / Hessian sweep; its P-step sums come from k_em_p_mixed
+     * (FP32 cells, FP64 across chunks). */
     int Sq = 1, Sp = 1;
     cudaError_t e;
     const bool mixed = (h->flags & ADMIX_FLAG_MIXED) != 0;
@@ -993,6 +996,7 @@ static void set_plans(admix_ctx *h, int sms_eff)
     h->sp = plan_sweep_p(h->K, h->I, h->J, sms_eff, h->cap_sp);
     h->sqm = plan_sweep_q_mixed(h->K, h->I, h->J, sms_eff, h->cap_sqm);
     h->spm = plan_sweep_p_mixed(h->K, h->I, h->J, sms_eff, h->cap_spm);
+    h->epm = plan_em_p_mixed(h->K, h->I, h->J, sms_eff, h->cap_spm * (h->K + 3) / 4);
     h->llm = plan_loglik_mixed(h->K, h->I, h->J, sms_eff, h->cap_llm);
     if (h->iter_graph) { cudaGraphExecDestroy(h->iter_graph); h->iter_graph = nullptr; }
     if (h->iter_graph_def) { cudaGraphDestroy(h->iter_graph_def); h->iter_graph_def = nullptr; }

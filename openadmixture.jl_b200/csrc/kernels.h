@@ -95,7 +95,9 @@ cudaError_t launch_sweep_q_mixed(int K, const uint8_t *bed, int64_t I, int64_t J
 size_t sweep_q_mixed_pkg_bytes(int K, int64_t J);
 
 SweepPlan plan_sweep_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax = INT64_MAX);
-/* The mixed P sweep first builds its per-chunk Q packages in pkg (sweep_p_mixed_pkg_bytes).
+SweepPlan plan_em_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax = INT64_MAX);
+/* The mixed P sweep first builds its per-chunk Q packages in pkg (sweep_p_mixed_pkg_bytes); pl: of plan_sweep_p_mixed
+ * (mode 0) or plan_em_p_mixed (mode 1).
  * mode 0: gradient / Hessian rows (T + K); mode 1: the EM P-step's two sums (2K, k_emp_finalize). */
 cudaError_t launch_sweep_p_mixed(int K, int mode, const uint8_t *bed, int64_t I, int64_t J, int64_t pitch,
                                  const double *q, const double *p, const SweepPlan &pl, double *out, int *err,

@@ -735,7 +735,7 @@ k_sweep_q_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
  *              added into FP64;
  * and per cell on the CUDA cores the code (from the thread's own genotype word), one reciprocal,
  * C, dz and its BF16 split.  The Q-derived tiles of each chunk (QQ in BF16, Q split into TF32
- * hi / lo, the gradient B blocks, q in FP32 for the EM mode) are built once per sweep by
+ * hi / lo, the gradient B blocks, q in FP32 for the EM sums) are built once per sweep by
  * k_p_pack and fetched with one bulk copy per chunk. */
 
 constexpr int MP_IC = 32;          /* individuals per chunk = 2 BF16 MMA K-steps */
@@ -758,7 +758,7 @@ struct MP {
     static constexpr uint32_t QB_BYTES = MP_IC * 2 * KP * 4;    /* TF32 Q chunk [hi | lo] */
     static constexpr uint32_t DGB_BYTES = NDG * MP_IC * 2;      /* one BF16 B block of the gradient MMAs */
     static constexpr int QS = MP_IC + 4;                        /* FP32 q row stride (floats) */
-    /* package: [QQ | TF32 Q | FP32 q (EM mode) | 1 - sum q | gradient blocks [q_hi | q_lo], [q_hi | 0]] */
+    /* package: [QQ | TF32 Q | FP32 q (EM sums) | 1 - sum q | gradient blocks [q_hi | q_lo], [q_hi | 0]] */
     static constexpr uint32_t PK_QB = B_BYTES;
     static constexpr uint32_t PK_QF = PK_QB + QB_BYTES;
     static constexpr uint32_t PK_S = PK_QF + K * QS * 4;         /* 1 - sum_k q_k per individual */
@@ -883,32 +883,51 @@ __device__ __forceinline__ uint2 col_load32(const uint8_t *__restrict__ bed, int
                  : make_uint2(0x55555555u, 0x55555555u);
 }
 
-/* Warp roles as in the Q sweep: warps 0-3 producers (thread = SNP row), warp 4 controller.
- *
- * EMS = true is the EM P-step of em_p! (algorithms_inner.jl:108-141, loops.jl:700-721) on the
- * same pipeline: per SNP the two sums sum_i nm g q_k / qp and sum_i nm (2-g) q_k / (1-qp)
- * (rows of 2K, the FP64 EM sweep's layout, finalised by k_emp_finalize), with no Hessian tile,
- * MMAs or drains; a package slot is handed back once the four producer warps have read it. */
+/* this thread's row of the TF32 P tile at pa and of the (1-P) tile that follows, from SNP j's p */
+template <int K>
+__device__ __forceinline__ void stage_p_rows(uint8_t *pa, const double *__restrict__ p, int64_t j, bool valid, int row)
+{
+    using C = MP<K>;
+    uint8_t *pb = pa + C::PA_BYTES;
+#pragma unroll
+    for (int f = 0; f < C::KP; f += 4) {
+        float hv[4], lv[4], hb[4], lb[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            hv[e] = lv[e] = hb[e] = lb[e] = 0.f;
+            if (f + e < K) {
+                const double pv = valid ? p[(size_t)K * j + f + e] : 0.5;
+                tf32_split((float)pv, hv[e], lv[e]);
+                tf32_split((float)(1.0 - pv), hb[e], lb[e]);
+            }
+        }
+        *(float4 *)(pa + kmaj_off(row, f, C::PA_LBO)) = make_float4(hv[0], hv[1], hv[2], hv[3]);
+        *(float4 *)(pa + kmaj_off(row, C::KP + f, C::PA_LBO)) = make_float4(lv[0], lv[1], lv[2], lv[3]);
+        *(float4 *)(pb + kmaj_off(row, f, C::PA_LBO)) = make_float4(hb[0], hb[1], hb[2], hb[3]);
+        *(float4 *)(pb + kmaj_off(row, C::KP + f, C::PA_LBO)) = make_float4(lb[0], lb[1], lb[2], lb[3]);
+    }
+}
+
+/* Warp roles as in the Q sweep: warps 0-3 producers (thread = SNP row), warp 4 controller. */
 constexpr int MP_CTA = MP_THREADS + 32;
 
-template <int K, bool EMS>
+template <int K>
 __global__ void __launch_bounds__(MP_CTA, (K <= 10 ? 3 : 2))
 k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pitch,
                 const uint8_t *__restrict__ pkg, const double *__restrict__ p, int64_t islice,
                 double *__restrict__ out, int *__restrict__ err)
 {
     using C = MP<K>;
-    constexpr int T = C::T, N = C::N, E = EMS ? 2 * K : C::E;
+    constexpr int T = C::T, N = C::N, E = C::E;
     extern __shared__ __align__(1024) uint8_t smraw[];
     uint8_t *sm = (uint8_t *)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
     /* qp ready, qp consumed (4 warps), A tiles written (4 warps), the chunk's MMAs done, package
-     * landed [3], package read (4 warps, EM sums only) [3], first half of the A tiles written (4
-     * warps), the first K-step's MMAs done */
-    __shared__ uint64_t mbar[6 + 2 * MP_NPKG];
+     * landed [3], first half of the A tiles written (4 warps), the first K-step's MMAs done */
+    __shared__ uint64_t mbar[6 + MP_NPKG];
     __shared__ uint32_t tmem_holder;
     __shared__ volatile int abort_flag;
     uint64_t *bar_qp = &mbar[0], *bar_qfree = &mbar[1], *bar_afull = &mbar[2], *bar_h = &mbar[3], *bar_p = &mbar[4];
-    uint64_t *bar_read = &mbar[4 + MP_NPKG], *bar_ahalf = &mbar[4 + 2 * MP_NPKG], *bar_h0 = &mbar[5 + 2 * MP_NPKG];
+    uint64_t *bar_ahalf = &mbar[4 + MP_NPKG], *bar_h0 = &mbar[5 + MP_NPKG];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool producer = warp < 4;
@@ -930,33 +949,13 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
         mbar_init(bar_afull, 4);
         mbar_init(bar_h, 1);
         for (int b = 0; b < MP_NPKG; ++b) mbar_init(&bar_p[b], 1);
-        for (int b = 0; b < MP_NPKG; ++b) mbar_init(&bar_read[b], 4);
         mbar_init(bar_ahalf, 4);
         mbar_init(bar_h0, 1);
         abort_flag = 0;
         mbar_fence_init();
     }
     code_table_init((float4 *)(sm + C::OFF_TAB), tid, MP_CTA);
-    if (producer) {   /* this thread's rows of the TF32 P and (1-P) tiles */
-        float hv[C::KP], lv[C::KP], hb[C::KP], lb[C::KP];
-#pragma unroll
-        for (int k = 0; k < C::KP; ++k) {
-            hv[k] = lv[k] = hb[k] = lb[k] = 0.f;
-            if (k < K) {
-                const double pv = valid ? p[(size_t)K * j + k] : 0.5;
-                tf32_split((float)pv, hv[k], lv[k]);
-                tf32_split((float)(1.0 - pv), hb[k], lb[k]);
-            }
-        }
-        uint8_t *pa = sm + C::OFF_PA, *pb = pa + C::PA_BYTES;
-#pragma unroll
-        for (int f = 0; f < C::KP; f += 4) {
-            *(float4 *)(pa + kmaj_off(tid, f, C::PA_LBO)) = make_float4(hv[f], hv[f + 1], hv[f + 2], hv[f + 3]);
-            *(float4 *)(pa + kmaj_off(tid, C::KP + f, C::PA_LBO)) = make_float4(lv[f], lv[f + 1], lv[f + 2], lv[f + 3]);
-            *(float4 *)(pb + kmaj_off(tid, f, C::PA_LBO)) = make_float4(hb[f], hb[f + 1], hb[f + 2], hb[f + 3]);
-            *(float4 *)(pb + kmaj_off(tid, C::KP + f, C::PA_LBO)) = make_float4(lb[f], lb[f + 1], lb[f + 2], lb[f + 3]);
-        }
-    }
+    if (producer) stage_p_rows<K>(sm + C::OFF_PA, p, j, valid, tid);
     fence_async_smem();
     tc_fence_before_sync();
     __syncthreads();
@@ -1003,12 +1002,11 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
                                                                          bbase + C::PK_DG, ks, (c % MX_DRAIN != 0) ? 1u : 0u);
         };
         for (int c = 0; c < nchunk && ok; ++c) {
-            if constexpr (!EMS) {   /* the first K-step (individuals 0-15) as soon as it is written */
-                if (wait(bar_ahalf, (uint32_t)(c & 1)) && leader) {
-                    tc_fence_after_sync();
-                    issue_ks(c, 0);
-                    tc_commit(bar_h0);
-                }
+            /* the first K-step (individuals 0-15) as soon as it is written */
+            if (wait(bar_ahalf, (uint32_t)(c & 1)) && leader) {
+                tc_fence_after_sync();
+                issue_ks(c, 0);
+                tc_commit(bar_h0);
             }
             if (c + 1 < nchunk) {
                 const int cn = c + 1;
@@ -1018,14 +1016,6 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
                     issue_qp_p<K>(tmem, sm + C::OFF_PA, sm + C::OFF_PKG + (cn % MP_NPKG) * C::PKG + C::PK_QB);
                     tc_commit(bar_qp);
                 }
-            }
-            if constexpr (EMS) {
-                /* slot c % 3's (c / 3)-th reading; its next one needs the copy issued here */
-                if (c + MP_NPKG < nchunk && wait(&bar_read[c % MP_NPKG], (uint32_t)((c / MP_NPKG) & 1))) {
-                    fence_async_smem();
-                    copy_pkg(c + MP_NPKG);
-                }
-                continue;
             }
             /* the second K-step once the producers wrote the rest of the chunk's A tiles */
             if (wait(bar_afull, (uint32_t)(c & 1)) && leader) {
@@ -1045,28 +1035,17 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
         uint2 gcur = make_uint2(0x55555555u, 0x55555555u), gnext = gcur;
         if (nchunk > 0) gcur = col_load32(bed, pitch, j, valid, ia);
         if (nchunk > 1) gnext = col_load32(bed, pitch, j, valid, ia + MP_IC);
-        /* gradient sum_i dz q_k (EM mode: sum_i nm g q_k / qp), Hessian diagonal, and the EM mode's
-         * second sums */
         uint32_t dst = dither_seed(j, blockIdx.y);   /* rounding dither of this row's Hessian weights */
-        double gd[K], dd[EMS ? 1 : K], hd[EMS ? K : 1];
+        double gd[K], dd[K];                          /* gradient sum_i dz q_k, Hessian diagonal */
 #pragma unroll
-        for (int k = 0; k < K; ++k) gd[k] = 0.0;
-#pragma unroll
-        for (int k = 0; k < (EMS ? 1 : K); ++k) dd[k] = 0.0;
-#pragma unroll
-        for (int k = 0; k < (EMS ? K : 1); ++k) hd[k] = 0.0;
+        for (int k = 0; k < K; ++k) gd[k] = dd[k] = 0.0;
         /* the last chunk whose MMAs completed: its Hessian diagonal (columns 0..K-1 of the Hessian
          * accumulator, cleared for the next chunk) and its gradient sums, into FP64 */
-        auto drain_dg = [&]() {
-            if constexpr (!EMS) drain_chunk<K, C::NDG>(tmem + lane_base, C::COL_H, C::COL_DG, dd, gd);
-        };
+        auto drain_dg = [&]() { drain_chunk<K, C::NDG>(tmem + lane_base, C::COL_H, C::COL_DG, dd, gd); };
         for (int c = 0; c < nchunk && ok; ++c) {
-            const uint8_t *pk = sm + C::OFF_PKG + (c % MP_NPKG) * C::PKG;
-            const float *Qf = (const float *)(pk + C::PK_QF);
-            const float2 *Sres = (const float2 *)(pk + C::PK_S);
-            if constexpr (!EMS) {   /* chunk c-1's first K-step MMAs are done: the A tiles' first half is free */
-                if (c > 0 && !wait(bar_h0, (uint32_t)((c - 1) & 1))) break;
-            }
+            const float2 *Sres = (const float2 *)(sm + C::OFF_PKG + (c % MP_NPKG) * C::PKG + C::PK_S);
+            /* chunk c-1's first K-step MMAs are done: the A tiles' first half is free */
+            if (c > 0 && !wait(bar_h0, (uint32_t)((c - 1) & 1))) break;
             /* qp / om of the chunk's 32 individuals, read in two halves of 16 columns
              * (individuals 0-15, then 16-31) to keep the producer within its registers */
             uint32_t rq[16], ro[16];
@@ -1076,11 +1055,6 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
             tmem_ld16_raw(tmem + lane_base + C::COL_OM, ro);
             tmem_wait_ld();
             if (!wait(&bar_p[c % MP_NPKG], (uint32_t)((c / MP_NPKG) & 1))) break;
-            float2 gk[K], hk[EMS ? K : 1];
-#pragma unroll
-            for (int k = 0; k < K; ++k) gk[k] = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < (EMS ? K : 1); ++k) hk[k] = make_float2(0.f, 0.f);
 #pragma unroll
             for (int kc = 0; kc < 4; ++kc) {
                 if (kc == 2) {   /* the second half of the columns; then the qp columns are free */
@@ -1093,7 +1067,6 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
                     if (lane == 0) mbar_arrive(bar_qfree);
                 }
                 uint32_t cp[4], d0p[4], d1p[4];
-                float2 zz[4], z2s[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int m = kc * 4 + e;
@@ -1108,101 +1081,56 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
                     const float2 r1 = __fmul2_rn(om, rr), r2 = __fmul2_rn(qp, rr);
                     const float2 z1 = __fmul2_rn(make_float2(a.x, a.y), r1);
                     const float2 z2 = __fmul2_rn(make_float2(a.z, a.w), r2);
-                    if constexpr (EMS) {
-                        zz[e] = z1;                                             /* nm g / qp */
-                        z2s[e] = z2;                                            /* nm (2-g) / (1-qp) */
-                    } else {
-                        const float2 cw = __ffma2_rn(z1, r1, __fmul2_rn(z2, r2));   /* nm (g/qp^2 + (2-g)/(1-qp)^2) */
-                        const float2 dz = __ffma2_rn(z2, make_float2(-1.f, -1.f), z1);   /* nm (g/qp - (2-g)/(1-qp)) */
-                        cp[e] = pack_bf16x2_dither(cw.x, cw.y, dither_step(dst));
-                        /* dz = hi + lo in BF16: hi rounded to nearest, lo the BF16 of the remainder */
-                        const uint32_t h = pack_bf16x2(dz.x, dz.y);
-                        const float2 hf = make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xFFFF0000u));
-                        const float2 lr = __fadd2_rn(dz, make_float2(-hf.x, -hf.y));
-                        d0p[e] = h;
-                        d1p[e] = pack_bf16x2(lr.x, lr.y);
-                    }
+                    const float2 cw = __ffma2_rn(z1, r1, __fmul2_rn(z2, r2));   /* nm (g/qp^2 + (2-g)/(1-qp)^2) */
+                    const float2 dz = __ffma2_rn(z2, make_float2(-1.f, -1.f), z1);   /* nm (g/qp - (2-g)/(1-qp)) */
+                    cp[e] = pack_bf16x2_dither(cw.x, cw.y, dither_step(dst));
+                    /* dz = hi + lo in BF16: hi rounded to nearest, lo the BF16 of the remainder */
+                    const uint32_t h = pack_bf16x2(dz.x, dz.y);
+                    const float2 hf = make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xFFFF0000u));
+                    const float2 lr = __fadd2_rn(dz, make_float2(-hf.x, -hf.y));
+                    d0p[e] = h;
+                    d1p[e] = pack_bf16x2(lr.x, lr.y);
                 }
-                if constexpr (!EMS) {
-                    *(uint4 *)(At + kc * C::A_LBO + 16 * tid) = make_uint4(cp[0], cp[1], cp[2], cp[3]);
-                    *(uint4 *)(At + C::A_BYTES + kc * C::A_LBO + 16 * tid) = make_uint4(d0p[0], d0p[1], d0p[2], d0p[3]);
-                    *(uint4 *)(At + 2 * C::A_BYTES + kc * C::A_LBO + 16 * tid) = make_uint4(d1p[0], d1p[1], d1p[2], d1p[3]);
-                    if (kc == 1) {   /* as on the Q side: drain chunk c-1, then release the first K-step */
-                        if (c > 0 && wait(bar_h, (uint32_t)((c - 1) & 1))) {
-                            if (c % MX_DRAIN == 0) drain_dg();
-                            if (c % MX_HBLOCK == 0) {
-                                tc_fence_after_sync();
-                                hess_drain<K, N, T>(tmem + lane_base + C::COL_H,
-                                                    out + ((size_t)blockIdx.y * J + (valid ? j : 0)) * E, c == MX_HBLOCK, valid);
-                                tc_fence_before_sync();
-                            }
+                *(uint4 *)(At + kc * C::A_LBO + 16 * tid) = make_uint4(cp[0], cp[1], cp[2], cp[3]);
+                *(uint4 *)(At + C::A_BYTES + kc * C::A_LBO + 16 * tid) = make_uint4(d0p[0], d0p[1], d0p[2], d0p[3]);
+                *(uint4 *)(At + 2 * C::A_BYTES + kc * C::A_LBO + 16 * tid) = make_uint4(d1p[0], d1p[1], d1p[2], d1p[3]);
+                if (kc == 1) {   /* as on the Q side: drain chunk c-1, then release the first K-step */
+                    if (c > 0 && wait(bar_h, (uint32_t)((c - 1) & 1))) {
+                        if (c % MX_DRAIN == 0) drain_dg();
+                        if (c % MX_HBLOCK == 0) {
+                            tc_fence_after_sync();
+                            hess_drain<K, N, T>(tmem + lane_base + C::COL_H,
+                                                out + ((size_t)blockIdx.y * J + (valid ? j : 0)) * E, c == MX_HBLOCK, valid);
+                            tc_fence_before_sync();
                         }
-                        fence_async_smem();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_ahalf);
                     }
-                } else {
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const float4 q0 = *(const float4 *)(Qf + k * C::QS + kc * 8);
-                    const float4 q1 = *(const float4 *)(Qf + k * C::QS + kc * 8 + 4);
-                    gk[k] = __ffma2_rn(zz[0], make_float2(q0.x, q0.y), gk[k]);
-                    gk[k] = __ffma2_rn(zz[1], make_float2(q0.z, q0.w), gk[k]);
-                    gk[k] = __ffma2_rn(zz[2], make_float2(q1.x, q1.y), gk[k]);
-                    gk[k] = __ffma2_rn(zz[3], make_float2(q1.z, q1.w), gk[k]);
-                    hk[k] = __ffma2_rn(z2s[0], make_float2(q0.x, q0.y), hk[k]);
-                    hk[k] = __ffma2_rn(z2s[1], make_float2(q0.z, q0.w), hk[k]);
-                    hk[k] = __ffma2_rn(z2s[2], make_float2(q1.x, q1.y), hk[k]);
-                    hk[k] = __ffma2_rn(z2s[3], make_float2(q1.z, q1.w), hk[k]);
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_ahalf);
                 }
-                }
-            }
-            if constexpr (EMS) {   /* the package is read: hand its slot back */
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_read[c % MP_NPKG]);
-            }
-            if constexpr (EMS) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) gd[k] += (double)gk[k].x + (double)gk[k].y;
-#pragma unroll
-                for (int k = 0; k < K; ++k) hd[k] += (double)hk[k].x + (double)hk[k].y;
             }
             if (c + 1 < nchunk) {
                 gcur = gnext;
                 if (c + 2 < nchunk) gnext = col_load32(bed, pitch, j, valid, ia + (int64_t)(c + 2) * MP_IC);
             }
-            if constexpr (!EMS) {
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_afull);
-            }
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_afull);
         }
-        if constexpr (EMS) {
-            if (valid) {   /* a thread whose wait gave up writes NaN sums (and err is set) */
-                double *o = out + ((size_t)blockIdx.y * J + j) * E;
-                const double bad = __longlong_as_double(0x7ff8000000000000LL);
+        if (nchunk > 0 && wait(bar_h, (uint32_t)((nchunk - 1) & 1))) drain_dg();   /* the last chunk */
+        if (valid) {
+            double *o = out + ((size_t)blockIdx.y * J + j) * E;
 #pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    o[k] = ok ? gd[k] : bad;
-                    o[K + k] = ok ? hd[k] : bad;
-                }
-            }
-        } else {
-            if (nchunk > 0 && wait(bar_h, (uint32_t)((nchunk - 1) & 1))) drain_dg();   /* the last chunk */
-            if (valid) {
-                double *o = out + ((size_t)blockIdx.y * J + j) * E;
-#pragma unroll
-                for (int k = 0; k < K; ++k) o[T + k] = ok ? gd[k] : __longlong_as_double(0x7ff8000000000000LL);
-            }
+            for (int k = 0; k < K; ++k) o[T + k] = ok ? gd[k] : __longlong_as_double(0x7ff8000000000000LL);
         }
-        if constexpr (!EMS) {   /* the epilogue below writes the diagonal from these */
+        /* the epilogue below writes the diagonal from these */
 #pragma unroll
-            for (int k = 0; k < K; ++k) diag_keep[k] = dd[k];
-        }
+        for (int k = 0; k < K; ++k) diag_keep[k] = dd[k];
     }
     ok = __syncthreads_and(ok);
     if (!ok && tid == MP_THREADS) {
-        if constexpr (!EMS) { mbar_wait_bounded(bar_h0, 0u, 1024u); mbar_wait_bounded(bar_h0, 1u, 1024u); }
+        mbar_wait_bounded(bar_h0, 0u, 1024u);
+        mbar_wait_bounded(bar_h0, 1u, 1024u);
         mbar_wait_bounded(bar_h, 0u, 1024u);
         mbar_wait_bounded(bar_h, 1u, 1024u);
         mbar_wait_bounded(bar_qp, 0u, 1024u);
@@ -1211,7 +1139,7 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
     }
     __syncthreads();
     tc_fence_after_sync();
-    if (producer && !EMS) {
+    if (producer) {
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         if (nchunk > 0) {
 #pragma unroll
@@ -1243,6 +1171,260 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 4) tmem_dealloc_warp(tmem, C::NCOLS);
+}
+
+/* ===================================================================== EM sums of the P side
+ *
+ * The EM P-step of em_p! (algorithms_inner.jl:108-141, loops.jl:700-721): per SNP the two sums sum_i nm g q_k / qp and
+ * sum_i nm (2-g) q_k / (1-qp) (rows of 2K, the FP64 EM sweep's layout, finalised by k_emp_finalize), qp and 1-qp from
+ * the tensor cores as in the P sweep, the sums in FP32 pairs per chunk and in FP64 across chunks.
+ *
+ * Bound by the CUDA cores: per pair of cells 2 K packed FMAs, two reciprocals and the weights, against 16 K bytes of q
+ * read from shared memory by every thread that adds one SNP.  So a thread adds R = 2 SNPs (128 apart) per q that it reads
+ * up to K = 8 (above that its 4 R K sums do not fit its registers), the codes come from byte permutes instead of a
+ * shared-memory table, and the FP64 sums, touched once per chunk, stand in shared memory.  Three CTAs share an SM up to
+ * K = 7, two above, which then hold two chunks of qp in tensor memory each (K = 6, 1e9 cells: 1.30 ms, two CTAs 1.41; at
+ * K = 8 three spill: 16.2 ms for 1e10 cells, two 15.9).  With one SNP per thread, the table and the sums in registers
+ * the shared-memory loads took 71 % of the pipe and the spills went to L2: 19.2 ms for 1e10 cells at K = 8 (now 15.9),
+ * 1.48 for 1e9 at K = 5 (1.14), 3.84 for 1.2e9 at K = 12 (3.09). */
+constexpr int ME_NPKG = 3;
+
+__host__ __device__ constexpr int em_rows(int K) { return K <= 8 ? 2 : 1; }
+
+template <int K>
+struct ME {
+    using C = MP<K>;
+    static constexpr int R = em_rows(K);                        /* SNPs per thread: tile r holds SNPs 128 r .. of the CTA */
+    static constexpr int CTAS = K <= 7 ? 3 : 2, NB = K <= 7 ? 1 : 2;   /* CTAs per SM, chunks of qp in TMEM */
+    static constexpr uint32_t BUF = R * 64, NCOLS = NB * BUF;   /* TMEM: per chunk R x [qp 32 | om 32] columns */
+    /* of the P sweep's package: TF32 Q, FP32 q and 1 - sum q */
+    static constexpr uint32_t PKG = C::PK_DG - C::PK_QB, PK_QF = C::PK_QF - C::PK_QB, PK_S = C::PK_S - C::PK_QB;
+    static constexpr uint32_t OFF_PA = ME_NPKG * PKG;
+    static constexpr uint32_t OFF_SUM = OFF_PA + R * 2 * C::PA_BYTES;   /* double [R][2K][128] */
+    static constexpr uint32_t SMEM = OFF_SUM + R * 2 * K * 128 * 8 + 128;
+    static_assert(PKG % 16 == 0 && C::PK_QB % 16 == 0, "bulk copies need 16-byte alignment");
+};
+
+/* Codes of 8 individuals (2 bits each, low first) spread to 4 bits each */
+__device__ __forceinline__ uint32_t spread8(uint32_t w16)
+{
+    uint32_t x = (w16 | (w16 << 8)) & 0x00FF00FFu;
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;
+    return (x | (x << 2)) & 0x33333333u;
+}
+
+/* (nm g, nm (2-g)) of four cells from their codes, 4 bits each (sel's low half): byte permutes look up the high bytes of
+ * the BF16 values 0, 1 and 2 (a low byte is 0x80 for 1, else 0), which widen to FP32 by a shift */
+__device__ __forceinline__ void code_quad(uint32_t sel, float2 (&a)[2], float2 (&b)[2])
+{
+    const uint32_t lo = __byte_perm(0x00800000u, 0u, sel);
+    const uint32_t h1 = __byte_perm(0x403F0000u, 0u, sel), h2 = __byte_perm(0x003F0040u, 0u, sel);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const uint32_t u = __byte_perm(lo, h1, t ? 0x7362u : 0x5140u), v = __byte_perm(lo, h2, t ? 0x7362u : 0x5140u);
+        a[t] = make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+        b[t] = make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u));
+    }
+}
+
+template <int K>
+__global__ void __launch_bounds__(MP_CTA, ME<K>::CTAS)
+k_em_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pitch,
+             const uint8_t *__restrict__ pkg, const double *__restrict__ p, int64_t islice,
+             double *__restrict__ out, int *__restrict__ err)
+{
+    using C = MP<K>;
+    using M = ME<K>;
+    constexpr int R = M::R, NB = M::NB, E = 2 * K;
+    extern __shared__ __align__(1024) uint8_t smraw[];
+    uint8_t *sm = (uint8_t *)(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
+    /* qp of buffer b ready [2], consumed (4 warps) [2], package landed [3], package read (4 warps) [3] */
+    __shared__ uint64_t mbar[4 + 2 * ME_NPKG];
+    __shared__ uint32_t tmem_holder;
+    __shared__ volatile int abort_flag;
+    uint64_t *bar_qp = &mbar[0], *bar_qfree = &mbar[2], *bar_p = &mbar[4], *bar_read = &mbar[4 + ME_NPKG];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool producer = warp < 4;
+    const int64_t j0 = (int64_t)blockIdx.x * (128 * R) + tid;    /* this thread's SNPs: j0, j0 + 128 */
+    const int64_t ia = (int64_t)blockIdx.y * islice;    /* islice is a multiple of MP_IC */
+    const int64_t ib = min(I, ia + islice);
+    const int nchunk = (int)((ib - ia + MP_IC - 1) / MP_IC);
+    const uint8_t *pk0 = pkg + (size_t)(ia / MP_IC) * C::PKG + C::PK_QB;
+
+    if (warp == 4) tmem_alloc_warp(&tmem_holder, M::NCOLS);
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) mbar_init(&bar_qp[b], 1);
+        for (int b = 0; b < 2; ++b) mbar_init(&bar_qfree[b], 4);
+        for (int b = 0; b < ME_NPKG; ++b) mbar_init(&bar_p[b], 1);
+        for (int b = 0; b < ME_NPKG; ++b) mbar_init(&bar_read[b], 4);
+        abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (producer)
+        for (int r = 0; r < R; ++r)
+            stage_p_rows<K>(sm + M::OFF_PA + r * 2 * C::PA_BYTES, p, j0 + 128 * r, j0 + 128 * r < J, tid);
+    fence_async_smem();
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = tmem_holder;
+    bool ok = true;
+    auto wait = [&](uint64_t *b, uint32_t parity) -> bool {
+        if (!ok) return false;
+        for (uint32_t n = 0; n < MX_WAIT_LIMIT; ++n) {
+            if (mbar_try_wait(b, parity)) return true;
+            if ((n & 255u) == 255u && abort_flag) break;
+        }
+        ok = false;
+        abort_flag = 1;
+        atomicOr(err, 1);
+        return false;
+    };
+
+    if (!producer) {
+        /* ---------------------------------------------------------------- controller warp */
+        const bool leader = lane == 0;
+        auto copy_pkg = [&](int c) {
+            if (leader) {
+                mbar_arrive_expect_tx(&bar_p[c % ME_NPKG], M::PKG);
+                bulk_g2s(sm + (c % ME_NPKG) * M::PKG, pk0 + (size_t)c * C::PKG, M::PKG, &bar_p[c % ME_NPKG]);
+            }
+        };
+        for (int c = 0; c < min(nchunk, ME_NPKG); ++c) copy_pkg(c);
+        for (int c = 0; c < nchunk && ok; ++c) {
+            const int b = c % NB;
+            if (!wait(&bar_p[c % ME_NPKG], (uint32_t)((c / ME_NPKG) & 1))) break;
+            if (c >= NB && !wait(&bar_qfree[b], (uint32_t)(((c - NB) / NB) & 1))) break;   /* buffer b was read */
+            if (leader) {
+                tc_fence_after_sync();
+                for (int r = 0; r < R; ++r)
+                    issue_qp_p<K>(tmem + (uint32_t)(b * M::BUF + r * 64), sm + M::OFF_PA + r * 2 * C::PA_BYTES,
+                                  sm + (c % ME_NPKG) * M::PKG);
+                tc_commit(&bar_qp[b]);
+            }
+            __syncwarp();
+            /* chunk c-2's package is read: fetch chunk c+1 into its slot */
+            if (c >= 2 && c + 1 < nchunk) {
+                if (!wait(&bar_read[(c - 2) % ME_NPKG], (uint32_t)(((c - 2) / ME_NPKG) & 1))) break;
+                fence_async_smem();
+                copy_pkg(c + 1);
+            }
+        }
+    } else {
+        /* ---------------------------------------------------------------- producer warps */
+        const uint32_t my = tmem + ((uint32_t)(warp * 32) << 16);
+        uint2 gcur[R], gnext[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            gcur[r] = col_load32(bed, pitch, j0 + 128 * r, nchunk > 0 && j0 + 128 * r < J, ia);
+            gnext[r] = col_load32(bed, pitch, j0 + 128 * r, nchunk > 1 && j0 + 128 * r < J, ia + MP_IC);
+        }
+        /* the FP64 sums: sum_i nm g q_k / qp at slot k of tile r, sum_i nm (2-g) q_k / (1-qp) at slot K + k */
+        double *sums = (double *)(sm + M::OFF_SUM) + tid;
+#pragma unroll
+        for (int k = 0; k < R * E; ++k) sums[k * 128] = 0.0;
+        for (int c = 0; c < nchunk && ok; ++c) {
+            const uint8_t *pk = sm + (c % ME_NPKG) * M::PKG;
+            const float *Qf = (const float *)(pk + M::PK_QF);
+            const float4 *Sres = (const float4 *)(pk + M::PK_S);
+            const uint32_t buf = my + (uint32_t)((c % NB) * M::BUF);
+            uint32_t rq[R][4], ro[R][4];   /* qp / om of 4 individuals */
+            if (!wait(&bar_qp[c % NB], (uint32_t)((c / NB) & 1))) break;
+            if (!wait(&bar_p[c % ME_NPKG], (uint32_t)((c / ME_NPKG) & 1))) break;
+            tc_fence_after_sync();
+            auto load = [&](int s) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    tmem_ld4_raw(buf + 64u * r + 4u * s, rq[r]);
+                    tmem_ld4_raw(buf + 64u * r + 32u + 4u * s, ro[r]);
+                }
+            };
+            uint32_t cw[R];
+            float2 z1[R][2], z2[R][2];
+            auto weights = [&](int s) {
+                const float4 sr = Sres[s];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if ((s & 1) == 0) {
+                        const uint32_t w = (s < 4) ? gcur[r].x : gcur[r].y;
+                        cw[r] = spread8((s & 2) ? w >> 16 : w & 0xFFFFu);
+                    }
+                    float2 a[2], b[2];
+                    code_quad((s & 1) ? cw[r] >> 16 : cw[r], a, b);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const float2 qp = make_float2(__uint_as_float(rq[r][2 * t]), __uint_as_float(rq[r][2 * t + 1]));
+                        const float2 om = __fadd2_rn(make_float2(__uint_as_float(ro[r][2 * t]), __uint_as_float(ro[r][2 * t + 1])),
+                                                     t ? make_float2(sr.z, sr.w) : make_float2(sr.x, sr.y));
+                        const float2 pr = __fmul2_rn(qp, om);
+                        const float2 rr = make_float2(rcp_approx(pr.x), rcp_approx(pr.y));
+                        z1[r][t] = __fmul2_rn(a[t], __fmul2_rn(om, rr));   /* nm g / qp */
+                        z2[r][t] = __fmul2_rn(b[t], __fmul2_rn(qp, rr));   /* nm (2-g) / (1-qp) */
+                    }
+                }
+            };
+            load(0);
+            float2 gk[R][K], hk[R][K];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int k = 0; k < K; ++k) gk[r][k] = hk[r][k] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                tmem_wait_ld();
+#pragma unroll
+                for (int r = 0; r < R; ++r)   /* ties the values to the wait */
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) asm volatile("" : "+r"(rq[r][e]), "+r"(ro[r][e]));
+                weights(s);
+                if (s < 7) load(s + 1);
+                else {   /* the qp columns are read */
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bar_qfree[c % NB]);
+                }
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const float4 q4 = *(const float4 *)(Qf + k * C::QS + 4 * s);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        gk[r][k] = __ffma2_rn(z1[r][0], make_float2(q4.x, q4.y), gk[r][k]);
+                        hk[r][k] = __ffma2_rn(z2[r][0], make_float2(q4.x, q4.y), hk[r][k]);
+                        gk[r][k] = __ffma2_rn(z1[r][1], make_float2(q4.z, q4.w), gk[r][k]);
+                        hk[r][k] = __ffma2_rn(z2[r][1], make_float2(q4.z, q4.w), hk[r][k]);
+                    }
+                }
+            }
+            __syncwarp();   /* the package is read: hand its slot back */
+            if (lane == 0) mbar_arrive(&bar_read[c % ME_NPKG]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    sums[(r * E + k) * 128] += (double)gk[r][k].x + (double)gk[r][k].y;
+                    sums[(r * E + K + k) * 128] += (double)hk[r][k].x + (double)hk[r][k].y;
+                }
+                gcur[r] = gnext[r];
+                gnext[r] = col_load32(bed, pitch, j0 + 128 * r, c + 2 < nchunk && j0 + 128 * r < J, ia + (int64_t)(c + 2) * MP_IC);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (j0 + 128 * r < J) {   /* a thread whose wait gave up writes NaN sums (and err is set) */
+                double *o = out + ((size_t)blockIdx.y * J + j0 + 128 * r) * E;
+#pragma unroll
+                for (int k = 0; k < E; ++k) o[k] = ok ? sums[(r * E + k) * 128] : __longlong_as_double(0x7ff8000000000000LL);
+            }
+    }
+    ok = __syncthreads_and(ok);
+    if (!ok && tid == MP_THREADS) {
+        for (int b = 0; b < 2; ++b) { mbar_wait_bounded(&bar_qp[b], 0u, 1024u); mbar_wait_bounded(&bar_qp[b], 1u, 1024u); }
+        for (int b = 0; b < ME_NPKG; ++b) { mbar_wait_bounded(&bar_p[b], 0u, 1024u); mbar_wait_bounded(&bar_p[b], 1u, 1024u); }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 4) tmem_dealloc_warp(tmem, M::NCOLS);
 }
 
 /* ===================================================================== loglik on the tensor cores
@@ -1555,8 +1737,8 @@ template <int K>
 cudaError_t prepare_mixed_t()
 {
     cudaError_t e = cudaFuncSetAttribute(k_sweep_q_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MQ<K>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sweep_p_mixed<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MP<K>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sweep_p_mixed<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MP<K>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sweep_p_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MP<K>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_em_p_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ME<K>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loglik_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT<K>::SMEM);
     return e;
 }
@@ -1590,9 +1772,9 @@ cudaError_t launch_p_mixed_t(int mode, const uint8_t *bed, int64_t I, int64_t J,
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)pl.gx, (unsigned)pl.S);
     if (mode == 1)
-        k_sweep_p_mixed<K, true><<<grid, MP_CTA, MP<K>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
+        k_em_p_mixed<K><<<grid, MP_CTA, ME<K>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
     else
-        k_sweep_p_mixed<K, false><<<grid, MP_CTA, MP<K>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
+        k_sweep_p_mixed<K><<<grid, MP_CTA, MP<K>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
     return cudaGetLastError();
 }
 
@@ -1663,8 +1845,11 @@ int resident_t(int kind)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_q_mixed<K>, MQ_CTA, MQ<K>::SMEM);
         est = resident_est(k_sweep_q_mixed<K>, MQ_CTA, MQ<K>::SMEM, MQ<K>::NCOLS);
     } else if (kind == 1) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p_mixed<K, false>, MP_CTA, MP<K>::SMEM);
-        est = resident_est(k_sweep_p_mixed<K, false>, MP_CTA, MP<K>::SMEM, MP<K>::NCOLS);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p_mixed<K>, MP_CTA, MP<K>::SMEM);
+        est = resident_est(k_sweep_p_mixed<K>, MP_CTA, MP<K>::SMEM, MP<K>::NCOLS);
+    } else if (kind == 3) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_p_mixed<K>, MP_CTA, ME<K>::SMEM);
+        est = resident_est(k_em_p_mixed<K>, MP_CTA, ME<K>::SMEM, ME<K>::NCOLS);
     } else {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_loglik_mixed<K>, LT_CTA, LT<K>::SMEM);
         est = resident_est(k_loglik_mixed<K>, LT_CTA, LT<K>::SMEM, LT<K>::NCOLS);
@@ -1678,7 +1863,7 @@ int resident_t(int kind)
 
 int resident(int kind, int K, int fallback)
 {
-    static int cache[3][17] = {};
+    static int cache[4][17] = {};
     if (K < 1 || K > 16) return fallback;
     int &c = cache[kind][K];
     if (c <= 0) {
@@ -1742,6 +1927,13 @@ SweepPlan plan_sweep_q_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
 SweepPlan plan_sweep_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
 {
     return plan_rows(J, I, sms, resident(1, K, 3), (int64_t)MX_DRAIN * MP_IC, 4, smax);
+}
+
+/* One CTA per 128 R SNPs (R = ME<K>::R) and individual slice. */
+SweepPlan plan_em_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
+{
+    const int R = em_rows(K);
+    return plan_rows((J + R - 1) / R, I, sms, resident(3, K, 2), (int64_t)MP_IC, 8, smax);
 }
 
 /* One CTA per 128 SNPs and individual slice (slices are multiples of 32 individuals). */

@@ -145,6 +145,13 @@ __device__ __forceinline__ void tmem_ld16_raw(uint32_t taddr, uint32_t (&r)[16])
                  : "r"(taddr) : "memory");
 }
 
+/* the same, 4 columns */
+__device__ __forceinline__ void tmem_ld4_raw(uint32_t taddr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 /* 16 consecutive FP32 columns of this thread's TMEM lane from registers (32x32b shape); complete
