@@ -21,6 +21,7 @@
  * accumulator restarts every 128 of the reduction and the threads add it into FP32 registers,
  * so no FP32 partial sees more than 24 of the tensor core's accumulations.
  */
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -28,6 +29,8 @@
 #include "common.cuh"
 #include "synth.h"
 #include "tc05.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -242,6 +245,7 @@ constexpr uint32_t GT_WAIT = 1u << 22;              /* polls of a bounded wait *
 constexpr uint32_t GT_A = GT_M * GT_K * 2, GT_B = GT_N * GT_K * 2;
 constexpr uint32_t GT_STAGE = 2 * GT_A + 2 * GT_B;
 constexpr uint32_t GT_SMEM = 2 * GT_STAGE + 1024;
+constexpr uint32_t GT_PART = GT_M * GT_N * 4;       /* one block's FP32 sums */
 constexpr uint32_t GT_A_LBO = GT_M * 16, GT_B_LBO = GT_N * 16;
 
 /* 8 values as BF16 high parts (rounded to nearest) and the BF16 of the remainders, v = hi + lo, packed in pairs */
@@ -266,12 +270,19 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo
  * elements a thread).  128 threads that read each of their 48 elements where they converted it put 48 memory
  * latencies in series: the encoder's first layer on 20,000
  * individuals took 2.78 ms, its weight gradient on 4,096 2.27 ms; now 0.75 and 0.20.  Every wait is
- * bounded; a CTA whose wait runs out writes NaN into its tile (the failure shows in the loss). */
-template <class LA, class LB>
-__global__ void __launch_bounds__(GT_THREADS, 2)
+ * bounded; a CTA whose wait runs out writes NaN into its tile (the failure shows in the loss).
+ *
+ * CL > 1: a cluster of CL CTAs shares a tile.  Each takes nb blocks of GT_D slices at a time and leaves every block's
+ * sums in its shared memory; then each adds all CTAs' blocks for its 16 / CL of a thread's columns, in the order
+ * of the reduction, so the result is bit for bit that of one CTA.  A
+ * 256 x 256 weight gradient over 4,096 individuals (8 tiles) took one CTA per tile 176 us at the latency of its 128
+ * slices. */
+template <class LA, class LB, int CL>
+__global__ void __launch_bounds__(GT_THREADS, CL == 8 ? 1 : 2)
 k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *__restrict__ bias, int act,
-          const float *__restrict__ mask, float *__restrict__ C, int64_t ldc)
+          const float *__restrict__ mask, float *__restrict__ C, int64_t ldc, int nb)
 {
+    constexpr int NE = 16 / CL;          /* columns a thread owns in the end */
     extern __shared__ __align__(1024) uint8_t smraw[];
     uint8_t *sm = (uint8_t *)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t bar[2];          /* MMAs of the slice in stage s done */
@@ -302,17 +313,27 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
         ok = false;
         abort_flag = 1;
     };
-    float acc[16];
+    float acc[NE];
 #pragma unroll
-    for (int n = 0; n < 16; ++n) acc[n] = 0.f;
-    auto drain = [&]() {   /* the finished accumulation block into the FP32 registers */
+    for (int n = 0; n < NE; ++n) acc[n] = 0.f;
+    float *part = (float *)(sm + 2 * GT_STAGE) + tid;     /* element e of block slot b: part[(16 b + e) * GT_THREADS] */
+    auto drain = [&](int slot) {   /* the finished accumulation block into the FP32 registers or its slot */
         tc_fence_after_sync();
         float v[16];
         tmem_ld16(my_tmem, v);
+        if constexpr (CL == 1) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[e] += v[e];
+            for (int e = 0; e < 16; ++e) acc[e] += v[e];
+        } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) part[(16 * slot + e) * GT_THREADS] = v[e];
+        }
     };
-    const int nch = (int)((Kd + GT_K - 1) / GT_K);
+    const int nch = (int)((Kd + GT_K - 1) / GT_K), nblk = (nch + GT_D - 1) / GT_D;
+    const int rank = CL == 1 ? 0 : (int)blockIdx.z, rounds = CL == 1 ? 1 : (nblk + CL * nb - 1) / (CL * nb);
+    /* this CTA's slices of a round */
+    auto first = [&](int round) { return CL == 1 ? 0 : (round * CL + rank) * nb * GT_D; };
+    auto count = [&](int round) { return CL == 1 ? nch : max(0, min(nch - first(round), nb * GT_D)); };
     constexpr uint32_t idesc = idesc_bf16_f32(GT_M, GT_N);
     typename LA::Raw ra;
     typename LB::Raw rb;
@@ -324,52 +345,72 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
         A.load(ra, m0 + am, k0 + 8 * ag, M, Kd);
         if (hasb) B.load(rb, n0 + bn, k0 + 8 * bg, N, Kd);
     };
-    if (nch > 0) fetch(0);
-    for (int c = 0; c < nch; ++c) {
-        const int st = c & 1;
-        uint8_t *Ah = sm + st * GT_STAGE, *Al = Ah + GT_A, *Bh = Al + GT_A, *Bl = Bh + GT_B;
-        if (c >= 2) wait(&bar[st], (uint32_t)(((c - 2) >> 1) & 1));   /* stage st is free again */
-        const int64_t k0 = (int64_t)c * GT_K;
-        float v[8];
-        uint4 h, l;
-        A.values(v, ra, m0 + am, k0 + 8 * ag, M, Kd);
-        split8(v, h, l);
-        *(uint4 *)(Ah + ag * GT_A_LBO + 16 * am) = h;
-        *(uint4 *)(Al + ag * GT_A_LBO + 16 * am) = l;
-        if (hasb) {
-            B.values(v, rb, n0 + bn, k0 + 8 * bg, N, Kd);
+    if (count(0) > 0) fetch(first(0));
+    int n = 0;                                            /* slices so far */
+    for (int round = 0; round < rounds; ++round) {
+        const int c0 = first(round), len = count(round);
+        for (int i = 0; i < len; ++i, ++n) {
+            const int c = c0 + i, st = n & 1;
+            uint8_t *Ah = sm + st * GT_STAGE, *Al = Ah + GT_A, *Bh = Al + GT_A, *Bl = Bh + GT_B;
+            if (n >= 2) wait(&bar[st], (uint32_t)(((n - 2) >> 1) & 1));   /* stage st is free again */
+            const int64_t k0 = (int64_t)c * GT_K;
+            float v[8];
+            uint4 h, l;
+            A.values(v, ra, m0 + am, k0 + 8 * ag, M, Kd);
             split8(v, h, l);
-            *(uint4 *)(Bh + bg * GT_B_LBO + 16 * bn) = h;
-            *(uint4 *)(Bl + bg * GT_B_LBO + 16 * bn) = l;
-        }
-        if (c + 1 < nch) fetch(c + 1);
-        fence_async_smem();
-        if (c > 0 && c % GT_D == 0) {   /* the block ending at slice c-1: its MMAs done, into registers */
-            wait(&bar[(c - 1) & 1], (uint32_t)(((c - 1) >> 1) & 1));
-            if (ok) drain();
-        }
-        tc_fence_before_sync();
-        __syncthreads();
-        tc_fence_after_sync();
-        if (tid == 0 && ok) {
-            const uint32_t ah = smem_u32(Ah), al = smem_u32(Al), bh = smem_u32(Bh), bl = smem_u32(Bl);
-#pragma unroll
-            for (int ks = 0; ks < GT_K / 16; ++ks) {
-                const uint32_t ao = ks * 2 * GT_A_LBO, bo = ks * 2 * GT_B_LBO;
-                const uint32_t fresh = (c % GT_D == 0 && ks == 0) ? 0u : 1u;
-                tc_mma_bf16(tmem, umma_desc_kmajor(ah + ao, GT_A_LBO, 128), umma_desc_kmajor(bh + bo, GT_B_LBO, 128),
-                            idesc, fresh);
-                tc_mma_bf16(tmem, umma_desc_kmajor(al + ao, GT_A_LBO, 128), umma_desc_kmajor(bh + bo, GT_B_LBO, 128),
-                            idesc, 1u);
-                tc_mma_bf16(tmem, umma_desc_kmajor(ah + ao, GT_A_LBO, 128), umma_desc_kmajor(bl + bo, GT_B_LBO, 128),
-                            idesc, 1u);
+            *(uint4 *)(Ah + ag * GT_A_LBO + 16 * am) = h;
+            *(uint4 *)(Al + ag * GT_A_LBO + 16 * am) = l;
+            if (hasb) {
+                B.values(v, rb, n0 + bn, k0 + 8 * bg, N, Kd);
+                split8(v, h, l);
+                *(uint4 *)(Bh + bg * GT_B_LBO + 16 * bn) = h;
+                *(uint4 *)(Bl + bg * GT_B_LBO + 16 * bn) = l;
             }
-            tc_commit(&bar[st]);
+            if (i + 1 < len) fetch(c + 1);
+            else if (round + 1 < rounds && count(round + 1) > 0) fetch(first(round + 1));
+            fence_async_smem();
+            if (i > 0 && i % GT_D == 0) {   /* the block ending at the slice before: its MMAs done */
+                wait(&bar[(n - 1) & 1], (uint32_t)(((n - 1) >> 1) & 1));
+                if (ok) drain(i / GT_D - 1);
+            }
+            tc_fence_before_sync();
+            __syncthreads();
+            tc_fence_after_sync();
+            if (tid == 0 && ok) {
+                const uint32_t ah = smem_u32(Ah), al = smem_u32(Al), bh = smem_u32(Bh), bl = smem_u32(Bl);
+#pragma unroll
+                for (int ks = 0; ks < GT_K / 16; ++ks) {
+                    const uint32_t ao = ks * 2 * GT_A_LBO, bo = ks * 2 * GT_B_LBO;
+                    const uint32_t fresh = (i % GT_D == 0 && ks == 0) ? 0u : 1u;
+                    tc_mma_bf16(tmem, umma_desc_kmajor(ah + ao, GT_A_LBO, 128), umma_desc_kmajor(bh + bo, GT_B_LBO, 128),
+                                idesc, fresh);
+                    tc_mma_bf16(tmem, umma_desc_kmajor(al + ao, GT_A_LBO, 128), umma_desc_kmajor(bh + bo, GT_B_LBO, 128),
+                                idesc, 1u);
+                    tc_mma_bf16(tmem, umma_desc_kmajor(ah + ao, GT_A_LBO, 128), umma_desc_kmajor(bl + bo, GT_B_LBO, 128),
+                                idesc, 1u);
+                }
+                tc_commit(&bar[st]);
+            }
         }
-    }
-    if (nch > 0) {   /* the last block */
-        wait(&bar[(nch - 1) & 1], (uint32_t)(((nch - 1) >> 1) & 1));
-        if (ok) drain();
+        if (len > 0) {   /* the last block */
+            wait(&bar[(n - 1) & 1], (uint32_t)(((n - 1) >> 1) & 1));
+            if (ok) drain((len - 1) / GT_D);
+        }
+        if constexpr (CL > 1) {
+            cg::cluster_group cl = cg::this_cluster();
+            ok = __syncthreads_and(ok);
+            if (!ok)
+                for (int e = 0; e < 16 * nb; ++e) part[e * GT_THREADS] = __int_as_float(0x7fc00000);
+            cl.sync();
+            const int left = nblk - round * CL * nb;              /* blocks from this round on */
+            for (int r = 0; r < CL; ++r) {
+                const float *src = cl.map_shared_rank(part, r) + (size_t)rank * NE * GT_THREADS;
+                for (int slot = 0; slot < min(nb, left - r * nb); ++slot)
+#pragma unroll
+                    for (int e = 0; e < NE; ++e) acc[e] += src[(16 * slot + e) * GT_THREADS];
+            }
+            cl.sync();                                            /* the slots are read */
+        }
     }
     ok = __syncthreads_and(ok);
     if (!ok && tid == 0) {   /* give MMAs still in flight a bounded moment before the TMEM goes */
@@ -379,8 +420,8 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
     const int64_t m = m0 + 32 * (warp & 3) + (tid & 31);
     if (m < M) {
 #pragma unroll
-        for (int n = 0; n < 16; ++n) {
-            const int64_t col = n0 + col0 + n;
+        for (int n = 0; n < NE; ++n) {
+            const int64_t col = n0 + col0 + rank * NE + n;
             if (col >= N) break;
             float v = alpha * acc[n] + (bias ? bias[col] : 0.f);
             if (act) v = fmaxf(v, 0.f);
@@ -393,18 +434,57 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
     if (warp == 0) tmem_dealloc_warp(tmem, GT_N);
 }
 
+/* A tile per cluster of CL CTAs, each holding at most NB blocks' sums at a time */
+template <int CL, int NB, class LA, class LB>
+cudaError_t gemm_split(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *bias, int act,
+                       const float *mask, float *C, int64_t ldc, dim3 grid, int64_t nblk, cudaStream_t st)
+{
+    static bool ready = false;   /* the kernel's dynamic shared memory limit, set once per instantiation */
+    if (!ready) {
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<LA, LB, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(GT_SMEM + NB * GT_PART));
+        if (e != cudaSuccess) return e;
+        ready = true;
+    }
+    const int64_t rounds = (nblk + CL * NB - 1) / (CL * NB);
+    const int nb = (int)((nblk + CL * rounds - 1) / (CL * rounds));
+    grid.z = CL;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = CL;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(GT_THREADS);
+    cfg.dynamicSmemBytes = GT_SMEM + (size_t)nb * GT_PART;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_gemm_tc<LA, LB, CL>, A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, nb);
+}
+
 template <class LA, class LB>
 cudaError_t gemm(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *bias, int act,
                  const float *mask, float *C, int64_t ldc, cudaStream_t st)
 {
     static bool ready = false;   /* the kernel's dynamic shared memory limit, set once per instantiation */
     if (!ready) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<LA, LB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
         if (e != cudaSuccess) return e;
         ready = true;
     }
     dim3 grid((unsigned)((N + GT_N - 1) / GT_N), (unsigned)((M + GT_M - 1) / GT_M));
-    k_gemm_tc<LA, LB><<<grid, GT_THREADS, GT_SMEM, st>>>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc);
+    const int64_t tiles = (int64_t)grid.x * grid.y, nblk = (Kd + GT_K * GT_D - 1) / (GT_K * GT_D);
+    /* Few tiles leave most SMs idle.  Eight CTAs per tile (one per SM: 177 KB) as long as they are about one wave:
+     * encoder forward pass of 300 / 640 / 1,024 individuals (12 / 20 / 32 tiles, 33 blocks in its first layer) 91 / 133 /
+     * 180 us, with one CTA per tile 238 / 227 / 229, with two 172 / 168 / 168.  Two (two per SM) while those are at most
+     * one per SM: 2,048 individuals (64 tiles) 175 us against 230; at 128 tiles 307 against 233.  Two blocks are worth
+     * eight CTAs (40 individuals, second layer too: 86 -> 78 us); two CTAs need the blocks to pay for their rounds. */
+    if (tiles <= 24 && nblk >= 2)
+        return gemm_split<8, 4>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, grid, nblk, st);
+    if (tiles <= 74 && nblk >= 8)
+        return gemm_split<2, 2>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, grid, nblk, st);
+    k_gemm_tc<LA, LB, 1><<<grid, GT_THREADS, GT_SMEM, st>>>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, 0);
     return cudaGetLastError();
 }
 
