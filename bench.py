@@ -87,6 +87,7 @@ def run_pass_only(args):
     with oa.CuAdmixData(d, g, flags=flags) as d_cu:
         pid = {"loglik": N.ADMIX_PASS_LOGLIK, "q_sweep": N.ADMIX_PASS_QSWEEP, "p_sweep": N.ADMIX_PASS_PSWEEP,
                "q_qp": N.ADMIX_PASS_QQP, "p_qp": N.ADMIX_PASS_PQP, "em": N.ADMIX_PASS_EM}[args.pass_only]
+        d_cu.upload(oa.X, d.x)
         if pid in (N.ADMIX_PASS_QQP, N.ADMIX_PASS_PQP):   # give the QPs real sweep outputs
             d_cu.time_pass(N.ADMIX_PASS_QSWEEP if pid == N.ADMIX_PASS_QQP else N.ADMIX_PASS_PSWEEP, 1)
         ms = d_cu.time_pass(pid, max(1, args.steps))
