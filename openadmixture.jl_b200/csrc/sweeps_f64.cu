@@ -29,15 +29,17 @@
  * a cell's qp, reciprocal and weights are formed once and that the operands of 1,024 FMAs
  * are one load per lane, where a scalar loop needs a shared load per two FMAs. */
 
+/* Both are collectives of the whole warp: volatile, so that the compiler leaves each where every lane executes it even if
+ * only some lanes use the result, and callers reconverge (__syncwarp) after a branch that lanes take apart. */
 __device__ __forceinline__ void dmma_k8(double (&d)[4], const double (&a)[4], double b0, double b1)
 {
-    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
                  : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
 }
 __device__ __forceinline__ void dmma_k4(double (&d)[4], double a0, double a1, double b0)
 {
-    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3]) : "d"(a0), "d"(a1), "d"(b0));
 }
 
@@ -268,17 +270,19 @@ k_loglik_f64(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t Ib, 
                 for (int b = 0; b < IC / 8; ++b) {
                     double qp[4], f[4];
                     factors(b, qp, f);
-                    if (ok) continue;
+                    if (!ok) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        acc += log_call(f[e]);
-                        const uint32_t cc = (((e & 2) ? xb[b >> 1] : xa[b >> 1]) >> (16 * (b & 1) + 2 * (e & 1))) & 3u;
-                        const int64_t j = (e & 2) ? jb : ja, i = i0 + (int64_t)c * IC + 8 * b + 2 * t + (e & 1);
-                        if (mu && cc == 1u && j < J && i < I) {   /* loglikelihood_loop: the missing dosage imputed by mu_j */
-                            const double gm = __ldg(mu + j);
-                            acc += gm * log_call(qp[e]) + (2.0 - gm) * log_call(1.0 - qp[e]);
+                        for (int e = 0; e < 4; ++e) {
+                            acc += log_call(f[e]);
+                            const uint32_t cc = (((e & 2) ? xb[b >> 1] : xa[b >> 1]) >> (16 * (b & 1) + 2 * (e & 1))) & 3u;
+                            const int64_t j = (e & 2) ? jb : ja, i = i0 + (int64_t)c * IC + 8 * b + 2 * t + (e & 1);
+                            if (mu && cc == 1u && j < J && i < I) {   /* loglikelihood_loop: the missing dosage imputed by mu_j */
+                                const double gm = __ldg(mu + j);
+                                acc += gm * log_call(qp[e]) + (2.0 - gm) * log_call(1.0 - qp[e]);
+                            }
                         }
                     }
+                    __syncwarp();                            /* the next block's product is the whole warp's */
                 }
             }
             const int64_t bits = __double_as_longlong(prod);
@@ -438,6 +442,7 @@ k_sweep_q_f64(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pit
                     cell_general(qp[e], code[e], mu && ((e & 1) ? vb : va) && j < j1, mu + j, w.z1[e], w.z2[e], w.w1[e], w.w2[e]);
                 }
             }
+            __syncwarp();                                      /* the sums are the whole warp's products */
         };
         auto sums = [&](int b, const CellW &w) {
             const int bo = g * CS + 8 * b + 2 * t;
@@ -601,6 +606,7 @@ k_sweep_p_f64(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pit
                                  w.z1[e], w.z2[e], w.w1[e], w.w2[e]);
                 }
             }
+            __syncwarp();
             if (MODE == 0) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
