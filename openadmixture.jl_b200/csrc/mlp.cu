@@ -26,6 +26,7 @@
 #include <math.h>
 #include <stdint.h>
 #include "../../include/admix.h"
+#include "col_words.h"
 #include "common.cuh"
 #include "synth.h"
 #include "tc05.cuh"
@@ -551,18 +552,25 @@ cudaError_t colsum(const float *dY, int64_t M, int64_t N, float *db, cudaStream_
     return cudaGetLastError();
 }
 
+struct ColRead {
+    __device__ __forceinline__ uint32_t byte(const uint8_t *p) const { return __ldg(p); }
+    __device__ __forceinline__ uint32_t word(const uint8_t *p) const { return __ldg((const uint32_t *)p); }
+};
+
 /* closed-form P step from Q: p_kj = sum_i nm q_ki g_ij / (2 sum_i nm q_ki), clamped to
  * [1e-5, 1-1e-5] like project_p! (projections.jl:69-74).  A thread owns two SNPs, one in each half of its paired
  * FP32 sums; q is staged through shared memory 64 individuals at a time with each value twice, so a pair of cells
  * takes one paired FMA per cluster and sum and no duplication of the genotype factors, which a table gives per code
  * pair.  A missing cell adds zeros, so no thread branches on the genotype.  Each sum is the same per-k FP32 sequence
  * as a per-cell loop that skips the missing cells.  W = 8: columns aligned to 8 bytes; otherwise
- * aligned words, shifted.
+ * aligned words, shifted (col_words.h).
  * Bound: instruction issue at the few warps that J / 2 threads are (the sums of a SNP are serial chains over the
  * individuals).  I=20k, J=100k, K=8: 2.53 ms with one SNP a thread and a byte per load, 1.88 now; two pairs a
- * thread, or the clusters split over two threads, repeat the staging or the decoding and take 2.35 to 2.46. */
+ * thread, or the clusters split over two threads, repeat the staging or the decoding and take 2.35 to 2.46.
+ * Registers up to K = 8: as many as it takes; left to itself the compiler chose 72 with spills for K = 3 (4,001 x 1,003,
+ * unaligned columns: 150 us, 123 so).  Above, its own choice: K = 11 at 20,003 x 100,001 takes 2.66 ms, 3.42 with more. */
 template <int K, int W>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(64, K <= 8 ? 1 : 0)
 k_warm_p(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, int64_t J, const double *__restrict__ q,
          double *__restrict__ p)
 {
@@ -591,27 +599,19 @@ k_warm_p(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, int64_t J, c
         return (x | (x << 2)) & 0x33333333u;
     };
     /* the 16 bytes of 64 individuals of a column, missing past its end */
-    auto codes = [&](const uint8_t *col, int64_t i0, uint32_t (&w)[4]) {
+    auto codes = [&](const uint8_t *col, int64_t i0, int64_t limit, uint32_t (&w)[4]) {
         const int64_t b0 = i0 >> 2;
 #pragma unroll
         for (int v = 0; v < 4; ++v) w[v] = 0x55555555u;
-        if (b0 + 16 <= Ib) {
+        if (b0 + 16 <= limit) {
             if (W == 8) {
                 const uint2 x = __ldg((const uint2 *)(col + b0)), y = __ldg((const uint2 *)(col + b0) + 1);
                 w[0] = x.x; w[1] = x.y; w[2] = y.x; w[3] = y.y;
-            } else {   /* the aligned words that hold the 16 bytes, each with at least one of them */
-                const uint32_t mis = (uint32_t)((uintptr_t)(col + b0) & 3u);
-                const uint32_t *al = (const uint32_t *)(col + b0 - mis);
-                uint32_t x[5];
-#pragma unroll
-                for (int v = 0; v < 5; ++v) x[v] = (v < 4 || mis) ? __ldg(al + v) : 0u;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) w[v] = __funnelshift_r(x[v], x[v + 1], 8 * mis);
+            } else {
+                block_words(ColRead{}, col + b0, w);
             }
         } else {
-#pragma unroll
-            for (int n = 0; n < 16; ++n)
-                if (b0 + n < Ib) w[n >> 2] = (w[n >> 2] & ~(0xFFu << (8 * (n & 3)))) | ((uint32_t)__ldg(col + b0 + n) << (8 * (n & 3)));
+            block_bytes(ColRead{}, col, b0, Ib, w);
         }
     };
     /* this thread's q values of the next 64 individuals; 0 past I, which adds nothing whatever the codes there */
@@ -626,8 +626,10 @@ k_warm_p(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, int64_t J, c
         }
     };
     uint32_t wa[4], wb[4];
-    codes(ca, 0, wa);
-    codes(cb, 0, wb);
+    const int64_t limit = W == 8 ? Ib : word_limit(blockIdx.x == gridDim.x - 1, Ib);
+    const int64_t limit0 = W == 8 ? Ib : first_word_limit(blockIdx.x == 0, bed, limit);
+    codes(ca, 0, limit0, wa);
+    codes(cb, 0, limit0, wb);
     fetch(0);
     for (int64_t i0 = 0; i0 < I; i0 += 64) {
         __syncthreads();
@@ -637,8 +639,8 @@ k_warm_p(const uint8_t *__restrict__ bed, int64_t pitch, int64_t I, int64_t J, c
         uint32_t na[4] = {wa[0], wa[1], wa[2], wa[3]}, nb[4] = {wb[0], wb[1], wb[2], wb[3]};
         if (i0 + 64 < I) {
             fetch(i0 + 64);
-            codes(ca, i0 + 64, na);
-            codes(cb, i0 + 64, nb);
+            codes(ca, i0 + 64, limit, na);
+            codes(cb, i0 + 64, limit, nb);
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
