@@ -127,10 +127,15 @@ __device__ __forceinline__ bool cells_fast(const double (&qp)[4], const uint32_t
     return (odd & 0xF0000000) == 0;   /* qp and 1 - qp in [2^-255, 2): the reciprocals and the doubling are safe */
 }
 
-/* the general form: dosage g (the SNP's mean mu for a missing cell when imp) and a division each */
-__device__ __forceinline__ void cell_general(double qp, uint32_t code, bool imp, const double *mu, double &z1, double &z2,
+/* the general form: dosage g (the SNP's mean mu for a missing cell when imp) and a division each; all weights zero for a
+ * cell past the tile's columns (!in), whose placeholder coefficients a row may well take to qp = 0 or 1 */
+__device__ __forceinline__ void cell_general(double qp, uint32_t code, bool in, bool imp, const double *mu, double &z1, double &z2,
                                              double &w1, double &w2)
 {
+    if (!in) {
+        z1 = z2 = w1 = w2 = 0.0;
+        return;
+    }
     const bool miss = (code & 3u) == 1u, nm = !miss || imp;
     const double g = (miss && imp) ? __ldg(mu) : gval((int)(code & 3u));
     const double r1 = rcp_div(qp), r2 = rcp_div(1.0 - qp);
@@ -439,7 +444,7 @@ k_sweep_q_f64(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pit
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int64_t j = j0 + (int64_t)c * JC + 8 * b + 2 * t + (e >> 1);
-                    cell_general(qp[e], code[e], mu && ((e & 1) ? vb : va) && j < j1, mu + j, w.z1[e], w.z2[e], w.w1[e], w.w2[e]);
+                    cell_general(qp[e], code[e], j < j1, mu && ((e & 1) ? vb : va), mu + j, w.z1[e], w.z2[e], w.w1[e], w.w2[e]);
                 }
             }
             __syncwarp();                                      /* the sums are the whole warp's products */
@@ -602,8 +607,8 @@ k_sweep_p_f64(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pit
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int64_t j = (e & 1) ? jb : ja;
-                    cell_general(qp[e], code[e], mu && j < J && i0 + (int64_t)c * IC + 8 * b + 2 * t + (e >> 1) < i1, mu + j,
-                                 w.z1[e], w.z2[e], w.w1[e], w.w2[e]);
+                    cell_general(qp[e], code[e], i0 + (int64_t)c * IC + 8 * b + 2 * t + (e >> 1) < i1, mu && j < J, mu + j, w.z1[e], w.z2[e],
+                                 w.w1[e], w.w2[e]);
                 }
             }
             __syncwarp();
