@@ -457,7 +457,7 @@ static cudaError_t enq_sweep_p_mode(admix_ctx *h, int mode, int wq, int wp, int 
         double *out = h->parts_p + (size_t)j0 * row;
         if (mx) {
             const auto plan = mode == 2 ? plan_em_p_mixed : plan_sweep_p_mixed;
-            const SweepPlan pl = h->streamed ? block_plan(plan(h->K, h->I, nj, h->sms, INT64_MAX), (h->I + 31) / 32 * 32)
+            const SweepPlan pl = h->streamed ? block_plan(plan(h->K, h->I, nj, h->sms, 1), (h->I + 31) / 32 * 32)
                                              : mode == 2 ? h->epm : h->spm;
             return launch_sweep_p_mixed(h->K, mode == 2 ? 1 : 0, bed, h->I, nj, h->pitch, Qof(h, wq), P, pl, out,
                                         &h->sc->tc_err, h->pkg, h->st);

@@ -41,7 +41,7 @@ struct Carver {
     }
 };
 
-struct SweepPlan  { int gx = 1, S = 1; int64_t slice = 1; };
+struct SweepPlan  { int gx = 1, S = 1; int64_t slice = 1; int rows = 128; };   /* rows of a CTA */
 
 LoglikPlan plan_loglik(int64_t I, int64_t J, int sms);
 /* Slices of the second axis for CTAs of 128 rows, per_sm of which are resident per SM: whole waves, slices

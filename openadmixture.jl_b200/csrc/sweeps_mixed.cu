@@ -1181,21 +1181,24 @@ k_sweep_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t p
  *
  * Bound by the CUDA cores: per pair of cells 2 K packed FMAs, two reciprocals and the weights, against 16 K bytes of q
  * read from shared memory by every thread that adds one SNP.  So a thread adds R = 2 SNPs (128 apart) per q that it reads
- * up to K = 8 (above that its 4 R K sums do not fit its registers), the codes come from byte permutes instead of a
- * shared-memory table, and the FP64 sums, touched once per chunk, stand in shared memory.  Three CTAs share an SM up to
- * K = 7, two above, which then hold two chunks of qp in tensor memory each (K = 6, 1e9 cells: 1.30 ms, two CTAs 1.41; at
- * K = 8 three spill: 16.2 ms for 1e10 cells, two 15.9).  With one SNP per thread, the table and the sums in registers
+ * up to K = 8 (above that its 4 R K sums do not fit its registers) where there are enough of them (plan_em_p_mixed), the codes
+ * come from byte permutes instead of a shared-memory table, and the FP64 sums, touched once per chunk, stand in shared memory.
+ * With R = 2 three CTAs share an SM up to K = 7, two at K = 8, which then hold two chunks of qp in tensor memory each (K = 6, 1e9
+ * cells: 1.30 ms, two CTAs 1.41; at K = 8 three spill: 16.2 ms for 1e10 cells, two 15.9); with R = 1 three up to K = 8 (four
+ * were no faster).  With one SNP per thread, the table and the sums in registers
  * the shared-memory loads took 71 % of the pipe and the spills went to L2: 19.2 ms for 1e10 cells at K = 8 (now 15.9),
  * 1.48 for 1e9 at K = 5 (1.14), 3.84 for 1.2e9 at K = 12 (3.09). */
 constexpr int ME_NPKG = 3;
 
-__host__ __device__ constexpr int em_rows(int K) { return K <= 8 ? 2 : 1; }
+constexpr int EM_K2 = 8;           /* two SNPs per thread up to this K (plan_em_p_mixed says when) */
 
-template <int K>
+/* RR SNPs per thread: tile r holds SNPs 128 r .. of the CTA */
+template <int K, int RR>
 struct ME {
     using C = MP<K>;
-    static constexpr int R = em_rows(K);                        /* SNPs per thread: tile r holds SNPs 128 r .. of the CTA */
-    static constexpr int CTAS = K <= 7 ? 3 : 2, NB = K <= 7 ? 1 : 2;   /* CTAs per SM, chunks of qp in TMEM */
+    static constexpr int R = RR;
+    /* CTAs per SM, chunks of qp in TMEM */
+    static constexpr int CTAS = R == 1 ? (K <= EM_K2 ? 3 : 2) : (K <= 7 ? 3 : 2), NB = R == 2 && K <= 7 ? 1 : 2;
     static constexpr uint32_t BUF = R * 64, NCOLS = NB * BUF;   /* TMEM: per chunk R x [qp 32 | om 32] columns */
     /* of the P sweep's package: TF32 Q, FP32 q and 1 - sum q */
     static constexpr uint32_t PKG = C::PK_DG - C::PK_QB, PK_QF = C::PK_QF - C::PK_QB, PK_S = C::PK_S - C::PK_QB;
@@ -1227,14 +1230,14 @@ __device__ __forceinline__ void code_quad(uint32_t sel, float2 (&a)[2], float2 (
     }
 }
 
-template <int K>
-__global__ void __launch_bounds__(MP_CTA, ME<K>::CTAS)
+template <int K, int RR>
+__global__ void __launch_bounds__(MP_CTA, ME<K, RR>::CTAS)
 k_em_p_mixed(const uint8_t *__restrict__ bed, int64_t I, int64_t J, int64_t pitch,
              const uint8_t *__restrict__ pkg, const double *__restrict__ p, int64_t islice,
              double *__restrict__ out, int *__restrict__ err)
 {
     using C = MP<K>;
-    using M = ME<K>;
+    using M = ME<K, RR>;
     constexpr int R = M::R, NB = M::NB, E = 2 * K;
     extern __shared__ __align__(1024) uint8_t smraw[];
     uint8_t *sm = (uint8_t *)(((uintptr_t)smraw + 127) & ~(uintptr_t)127);
@@ -1738,7 +1741,9 @@ cudaError_t prepare_mixed_t()
 {
     cudaError_t e = cudaFuncSetAttribute(k_sweep_q_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MQ<K>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sweep_p_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MP<K>::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_em_p_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ME<K>::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_em_p_mixed<K, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ME<K, 1>::SMEM);
+    if constexpr (K <= EM_K2)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_em_p_mixed<K, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ME<K, 2>::SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loglik_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT<K>::SMEM);
     return e;
 }
@@ -1771,9 +1776,14 @@ cudaError_t launch_p_mixed_t(int mode, const uint8_t *bed, int64_t I, int64_t J,
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)pl.gx, (unsigned)pl.S);
-    if (mode == 1)
-        k_em_p_mixed<K><<<grid, MP_CTA, ME<K>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
-    else
+    if (mode == 1) {
+        if constexpr (K <= EM_K2)
+            if (pl.rows == 256) {
+                k_em_p_mixed<K, 2><<<grid, MP_CTA, ME<K, 2>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
+                return cudaGetLastError();
+            }
+        k_em_p_mixed<K, 1><<<grid, MP_CTA, ME<K, 1>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
+    } else
         k_sweep_p_mixed<K><<<grid, MP_CTA, MP<K>::SMEM, st>>>(bed, I, J, pitch, pkg, p, pl.slice, out, err);
     return cudaGetLastError();
 }
@@ -1848,8 +1858,12 @@ int resident_t(int kind)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_p_mixed<K>, MP_CTA, MP<K>::SMEM);
         est = resident_est(k_sweep_p_mixed<K>, MP_CTA, MP<K>::SMEM, MP<K>::NCOLS);
     } else if (kind == 3) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_p_mixed<K>, MP_CTA, ME<K>::SMEM);
-        est = resident_est(k_em_p_mixed<K>, MP_CTA, ME<K>::SMEM, ME<K>::NCOLS);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_p_mixed<K, 1>, MP_CTA, ME<K, 1>::SMEM);
+        est = resident_est(k_em_p_mixed<K, 1>, MP_CTA, ME<K, 1>::SMEM, ME<K, 1>::NCOLS);
+    } else if (kind == 4) {
+        constexpr int R = K <= EM_K2 ? 2 : 1;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_p_mixed<K, R>, MP_CTA, ME<K, R>::SMEM);
+        est = resident_est(k_em_p_mixed<K, R>, MP_CTA, ME<K, R>::SMEM, ME<K, R>::NCOLS);
     } else {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_loglik_mixed<K>, LT_CTA, LT<K>::SMEM);
         est = resident_est(k_loglik_mixed<K>, LT_CTA, LT<K>::SMEM, LT<K>::NCOLS);
@@ -1863,7 +1877,7 @@ int resident_t(int kind)
 
 int resident(int kind, int K, int fallback)
 {
-    static int cache[4][17] = {};
+    static int cache[5][17] = {};
     if (K < 1 || K > 16) return fallback;
     int &c = cache[kind][K];
     if (c <= 0) {
@@ -1929,11 +1943,20 @@ SweepPlan plan_sweep_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
     return plan_rows(J, I, sms, resident(1, K, 3), (int64_t)MX_DRAIN * MP_IC, 4, smax);
 }
 
-/* One CTA per 128 R SNPs (R = ME<K>::R) and individual slice. */
+/* One CTA per 256 SNPs (two per thread) and individual slice where that fills the GPU with CTAs of at least 24 chunks and pads
+ * the SNPs no further than tiles of 128 would; else per 128 SNPs.  P-step's part of an EM iteration in us, 128 / 256: K=5 I=20k
+ * J=50k 1271 / 1132, 10k x 20k 277 / 263 (29 chunks); 5k x 5k 58 / 61 (8 chunks), 1k x 10k 42 / 49, 100k x 300 112 / 145
+ * (512 rows for 384); a streamed block of 4,096 SNPs, whose slices are whole columns (16 CTAs): 10k x 16k 2611 / 3399. */
 SweepPlan plan_em_p_mixed(int K, int64_t I, int64_t J, int sms, int64_t smax)
 {
-    const int R = em_rows(K);
-    return plan_rows((J + R - 1) / R, I, sms, resident(3, K, 2), (int64_t)MP_IC, 8, smax);
+    const SweepPlan one = plan_rows(J, I, sms, resident(3, K, 2), (int64_t)MP_IC, 8, smax);
+    if (K > EM_K2) return one;
+    const int per_sm = resident(4, K, 2);
+    SweepPlan two = plan_rows((J + 1) / 2, I, sms, per_sm, (int64_t)MP_IC, 8, smax);
+    two.rows = 256;
+    const bool fills = 4 * (int64_t)two.gx * two.S >= 3 * (int64_t)sms * per_sm;
+    const bool tight = 33 * (int64_t)one.gx * one.rows >= 32 * (int64_t)two.gx * two.rows;
+    return fills && tight && two.slice >= 24 * MP_IC ? two : one;
 }
 
 /* One CTA per 128 SNPs and individual slice (slices are multiples of 32 individuals). */
