@@ -435,18 +435,21 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
     if (warp == 0) tmem_dealloc_warp(tmem, GT_N);
 }
 
+/* The dynamic shared memory limit belongs to the device, and callers may change devices and threads between two calls: set
+ * before every launch (0.2 us) instead of remembered. */
+template <class LA, class LB, int CL>
+cudaError_t allow_smem(size_t bytes)
+{
+    return cudaFuncSetAttribute(k_gemm_tc<LA, LB, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 /* A tile per cluster of CL CTAs, each holding at most NB blocks' sums at a time */
 template <int CL, int NB, class LA, class LB>
 cudaError_t gemm_split(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *bias, int act,
                        const float *mask, float *C, int64_t ldc, dim3 grid, int64_t nblk, cudaStream_t st)
 {
-    static bool ready = false;   /* the kernel's dynamic shared memory limit, set once per instantiation */
-    if (!ready) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<LA, LB, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(GT_SMEM + NB * GT_PART));
-        if (e != cudaSuccess) return e;
-        ready = true;
-    }
+    const cudaError_t e = allow_smem<LA, LB, CL>(GT_SMEM + NB * GT_PART);
+    if (e != cudaSuccess) return e;
     const int64_t rounds = (nblk + CL * NB - 1) / (CL * NB);
     const int nb = (int)((nblk + CL * rounds - 1) / (CL * rounds));
     grid.z = CL;
@@ -468,12 +471,6 @@ template <class LA, class LB>
 cudaError_t gemm(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *bias, int act,
                  const float *mask, float *C, int64_t ldc, cudaStream_t st)
 {
-    static bool ready = false;   /* the kernel's dynamic shared memory limit, set once per instantiation */
-    if (!ready) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<LA, LB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
-        if (e != cudaSuccess) return e;
-        ready = true;
-    }
     dim3 grid((unsigned)((N + GT_N - 1) / GT_N), (unsigned)((M + GT_M - 1) / GT_M));
     const int64_t tiles = (int64_t)grid.x * grid.y, nblk = (Kd + GT_K * GT_D - 1) / (GT_K * GT_D);
     /* Few tiles leave most SMs idle.  Eight CTAs per tile (one per SM: 177 KB) as long as they are about one wave:
@@ -485,6 +482,8 @@ cudaError_t gemm(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, cons
         return gemm_split<8, 4>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, grid, nblk, st);
     if (tiles <= 74 && nblk >= 8)
         return gemm_split<2, 2>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, grid, nblk, st);
+    const cudaError_t e = allow_smem<LA, LB, 1>(GT_SMEM);
+    if (e != cudaSuccess) return e;
     k_gemm_tc<LA, LB, 1><<<grid, GT_THREADS, GT_SMEM, st>>>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, 0);
     return cudaGetLastError();
 }
