@@ -271,11 +271,11 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo
  * elements a thread).  128 threads that read each of their 48 elements where they converted it put 48 memory
  * latencies in series: the encoder's first layer on 20,000
  * individuals took 2.78 ms, its weight gradient on 4,096 2.27 ms; now 0.75 and 0.20.  Every wait is
- * bounded; a CTA whose wait runs out writes NaN into its tile (the failure shows in the loss).
+ * bounded; a CTA whose wait runs out writes NaN into its tile, and the ReLU keeps NaN, so that the failure shows in the loss.
  *
  * CL > 1: a cluster of CL CTAs shares a tile.  Each takes nb blocks of GT_D slices at a time and leaves every block's
  * sums in its shared memory; then each adds all CTAs' blocks for its 16 / CL of a thread's columns, in the order
- * of the reduction, so the result is bit for bit that of one CTA.  A
+ * of the reduction, so the result is bit for bit that of one CTA (a CTA whose wait ran out leaves NaN in its slots).  A
  * 256 x 256 weight gradient over 4,096 individuals (8 tiles) took one CTA per tile 176 us at the latency of its 128
  * slices. */
 template <class LA, class LB, int CL>
@@ -425,7 +425,7 @@ k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float
             const int64_t col = n0 + col0 + rank * NE + n;
             if (col >= N) break;
             float v = alpha * acc[n] + (bias ? bias[col] : 0.f);
-            if (act) v = fmaxf(v, 0.f);
+            if (act && v <= 0.f) v = 0.f;                         /* NaN stays */
             if (mask && !(mask[m * ldc + col] > 0.f)) v = 0.f;
             C[m * ldc + col] = ok ? v : __int_as_float(0x7fc00000);
         }
