@@ -277,7 +277,7 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo
  * sums in its shared memory; then each adds all CTAs' blocks for its 16 / CL of a thread's columns, in the order
  * of the reduction, so the result is bit for bit that of one CTA (a CTA whose wait ran out leaves NaN in its slots).  A
  * 256 x 256 weight gradient over 4,096 individuals (8 tiles) took one CTA per tile 176 us at the latency of its 128
- * slices. */
+ * slices.  CL = 2 keeps the 64 registers of two CTAs per SM, but its blocks' slots (113 KB) leave room for one. */
 template <class LA, class LB, int CL>
 __global__ void __launch_bounds__(GT_THREADS, CL == 8 ? 1 : 2)
 k_gemm_tc(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, const float *__restrict__ bias, int act,
@@ -473,16 +473,20 @@ cudaError_t gemm(LA A, LB B, int64_t M, int64_t N, int64_t Kd, float alpha, cons
 {
     dim3 grid((unsigned)((N + GT_N - 1) / GT_N), (unsigned)((M + GT_M - 1) / GT_M));
     const int64_t tiles = (int64_t)grid.x * grid.y, nblk = (Kd + GT_K * GT_D - 1) / (GT_K * GT_D);
-    /* Few tiles leave most SMs idle.  Eight CTAs per tile (one per SM: 177 KB) as long as they are about one wave:
-     * encoder forward pass of 300 / 640 / 1,024 individuals (12 / 20 / 32 tiles, 33 blocks in its first layer) 91 / 133 /
-     * 180 us, with one CTA per tile 238 / 227 / 229, with two 172 / 168 / 168.  Two (two per SM) while those are at most
-     * one per SM: 2,048 individuals (64 tiles) 175 us against 230; at 128 tiles 307 against 233.  Two blocks are worth
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    /* Few tiles leave most SMs idle.  Eight CTAs per tile (one per SM: 177 KB) up to 4/3 of a wave, a sixth of the SMs' number of
+     * tiles: encoder forward pass of 300 / 640 / 1,024 individuals (12 / 20 / 32 tiles on 148 SMs, 33 blocks in its first layer)
+     * 91 / 133 / 180 us, with one CTA per tile 238 / 227 / 229, with two 172 / 168 / 168.  Two (one per SM as well: 113 KB) up to
+     * one wave: 2,048 individuals (64 tiles) 175 us against 230; at 128 tiles 307 against 233.  Two blocks are worth
      * eight CTAs (40 individuals, second layer too: 86 -> 78 us); two CTAs need the blocks to pay for their rounds. */
-    if (tiles <= 24 && nblk >= 2)
+    if (6 * tiles <= sms && nblk >= 2)
         return gemm_split<8, 4>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, grid, nblk, st);
-    if (tiles <= 74 && nblk >= 8)
+    if (2 * tiles <= sms && nblk >= 8)
         return gemm_split<2, 2>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, grid, nblk, st);
-    const cudaError_t e = allow_smem<LA, LB, 1>(GT_SMEM);
+    e = allow_smem<LA, LB, 1>(GT_SMEM);
     if (e != cudaSuccess) return e;
     k_gemm_tc<LA, LB, 1><<<grid, GT_THREADS, GT_SMEM, st>>>(A, B, M, N, Kd, alpha, bias, act, mask, C, ldc, 0);
     return cudaGetLastError();

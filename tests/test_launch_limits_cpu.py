@@ -56,3 +56,17 @@ def test_a_second_device_is_allowed_the_products_shared_memory(steps):
     for n in (300, 2048, 20000):                          # eight, two and one CTA per tile in the first layer
         for s in steps([n, 0, 148], [n, 1, 148], [n, 0, 148]):
             assert s["rc"] == [0, 0] and s["refused"] == 0, (n, s)
+
+
+def _first_layer(n, sms):
+    """CTAs per tile of the forward pass's first layer: 4 column tiles and 33 blocks of the reduction"""
+    tiles = 4 * -(-n // 128)
+    return 8 if 6 * tiles <= sms else 2 if 2 * tiles <= sms else 1
+
+
+def test_tiles_are_shared_by_the_devices_size(steps):
+    ns = (1, 128, 300, 768, 769, 1024, 2304, 2305, 4096)
+    assert [_first_layer(n, 148) for n in ns] == [8, 8, 8, 8, 2, 2, 2, 1, 1]
+    for sms in (148, 74, 296):
+        for n, s in zip(ns, steps(*[[n, 0, sms] for n in ns])):
+            assert s["rc"] == [0, 0] and s["cluster"][0] == _first_layer(n, sms), (n, sms)
