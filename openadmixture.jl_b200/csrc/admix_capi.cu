@@ -221,9 +221,14 @@ static int create_common(int64_t I, int64_t J, int32_t K, int32_t Q, const uint8
         mem.add(&h->bed, (size_t)h->pitch * J + 64);
     }
     mem.add(&h->xbuf, (size_t)4 * nx);
-    mem.add(&h->parts_q, (size_t)std::max(std::max(h->sq.S, (flags & ADMIX_FLAG_MIXED) ? h->sqm.S : 1),
-                                                  h->nblk) * I * E);
-    mem.add(&h->parts_p, (size_t)std::max(h->sp.S, (flags & ADMIX_FLAG_MIXED) ? h->spm.S : 1) * J * E);
+    /* Partial sums: slices x rows x entries.  The FP64 plans take as many slices as fill the GPU with CTAs of 128 rows (200k x
+     * 500k, K=8: 3 and 4, 0.9 GB beside 25 GB of genotypes; 20k x 60k, K=12: 14 and 5, 0.4 GB); a mixed handle needs
+     * theirs for the EM sums alone, whose rows are K and 2 K long instead of E. */
+    const bool mixed = (flags & ADMIX_FLAG_MIXED) != 0;
+    const int64_t row_q = mixed ? std::max<int64_t>(h->sqm.S * E, (int64_t)h->sq.S * K) : h->sq.S * E;
+    const int64_t row_p = mixed ? std::max<int64_t>(h->spm.S * E, (int64_t)h->sp.S * 2 * K) : h->sp.S * E;
+    mem.add(&h->parts_q, (size_t)(std::max<int64_t>(row_q, h->nblk * E) * I));
+    mem.add(&h->parts_p, (size_t)(row_p * J));
     mem.add(&h->U, (size_t)nx * Q);
     mem.add(&h->V, (size_t)nx * Q);
     mem.add(&h->vt, (size_t)K * K);
