@@ -62,7 +62,7 @@ extern "C" int admix_loglik_dev_noalloc(const uint8_t *d_bed, int64_t I, int64_t
     if (dev < 0 || dev >= kMaxDevices) return noalloc_fail(ADMIX_ERR_UNSUPPORTED, "device index beyond 63");
     const LoglikPlan pl = plan_loglik(I, J, sms);
     /* the documented size limit, 1024 individuals per slot of the scratch; the plan itself needs no more
-     * slots than two per SM */
+     * slots than four per SM */
     const int64_t groups = ((I + 3) / 4 + 255) / 256;
     if (groups > ADMIX_NOALLOC_MAX_PARTIALS || pl.gx > ADMIX_NOALLOC_MAX_PARTIALS) {
         char buf[200];

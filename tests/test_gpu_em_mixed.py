@@ -1,5 +1,5 @@
-"""The Float32 form's EM P-step at the edges of its kernel: 128 or 256 SNPs a CTA (two per thread up to K = 8), chunks of
-32 individuals, one chunk of qp in tensor memory up to K = 7 and two above.  Reference: the oracle's em_p.
+"""The Float32 form's EM P-step on small cohorts, at the edges of its tiles of 128 SNPs and chunks of 32 individuals
+(tiles of 256 SNPs need more of both).  Reference: the oracle's em_p.
 
 Tolerance on p in [0, 1]: qp and 1 - qp carry 2^-21 relative from the split TF32 products (all terms are positive) and the
 tensor core's FP32 accumulation, the reciprocal 2^-22, five FP32 products and an FP32 sum of 16 terms 21 * 2^-24: below

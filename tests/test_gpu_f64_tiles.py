@@ -1,6 +1,6 @@
 """The FP64 sweeps and log-likelihood at the edges of their tiles: 128 rows a CTA, 16 a warp, chunks of 32
 columns (16 above K = 8), 8-column pair tiles and 4-cluster products.  Reference: the oracle, at the
-1e-10 that the parity tests use (sums of at most 1e3 terms in another order: a few hundred ulp), and for points
+1e-10 that the parity tests use, and for points
 where qp is exactly 0 or 1 the same formulas in numpy."""
 import ctypes as C
 

@@ -1,5 +1,5 @@
-"""The learned start's kernels at the sizes and alignments their branches turn on: sketch blocks of 32 individuals and
-steps of 16 SNPs (rows of any alignment), columns at any pitch, SNP pairs, 64-individual chunks, and products whose
+"""The learned start's kernels at ragged sizes and alignments: sketches whose blocks of 4 individuals and strides of 256
+SNPs do not come out even, columns at any pitch, SNP pairs, 64-individual chunks, and products whose
 input rows are not 8-byte aligned."""
 import sys
 from pathlib import Path
